@@ -168,6 +168,9 @@ int ensure_tables(int device)
   ADV_CUDA(adv::upload_tables_diag(td, tf));
   ADV_CUDA(adv::upload_tables_implicit(td, tf));
   ADV_CUDA(adv::upload_tables_batch(td, tf));
+  ADV_CUDA(adv::upload_tables_fx_a(td, tf));
+  ADV_CUDA(adv::upload_tables_fx_b(td, tf));
+  ADV_CUDA(adv::upload_tables_fx_c(td, tf));
   ADV_CUDA(adv::upload_tables_gauss64(td, tf));
   ADV_CUDA(adv::upload_tables_gauss32(td, tf));
   g_tables_uploaded[device] = true;
@@ -335,6 +338,8 @@ adv::StageArgs base_args(const adv_handle &h, double t, int prec = -1)
   A.skewf    = (float)h.cfg.factor_skew;
   A.has_skew = h.cfg.factor_skew != 0.0;
   A.cell_geo = geo64 ? (const void *)h.d_cell_geo64 : h.d_cell_geo;
+  A.fx_ok    = h.fx_ok;
+  A.cell_exp = h.d_cell_exp;
   A.t        = t;
   A.ex       = h.diag.ex;
   const double s = time_factor(h, t);
@@ -594,6 +599,19 @@ int create_handle(const adv_config *cfg, int z_begin, int z_end, adv_handle **ou
         h->cv[d] = g.cv[d], h->P[d] = g.P[d], h->M[d] = g.M[d];
       const bool fp64 = h->cfg.precision == ADV_PRECISION_FP64;
       const bool both = h->cfg.precision == ADV_PRECISION_FP32_INCREMENT;
+      // the block fixed-point stages: every form with an FP64 operator
+      h->fx_ok = g.fx_ok && (fp64 || both);
+      if (h->fx_ok && !g.cell_exp.empty())
+        {
+          const size_t nb = g.cell_exp.size() * sizeof(int);
+          if ((e = cudaMalloc(&h->d_cell_exp, nb)) != cudaSuccess ||
+              (e = cudaMemcpy(h->d_cell_exp, g.cell_exp.data(), nb, cudaMemcpyHostToDevice)) != cudaSuccess)
+            {
+              rc = cuda_fail(e, "cell exponents");
+              break;
+            }
+          h->device_bytes += (int64_t)nb;
+        }
       if (!g.cell.empty())
         {
           rc = fp64 ? upload_array<double>(g.cell, &h->d_cell_geo, h->device_bytes)
@@ -718,6 +736,7 @@ int adv_destroy(adv_handle *h)
     return ADV_OK;
   cudaFree(h->d_cell_geo);
   cudaFree(h->d_cell_geo64);
+  cudaFree(h->d_cell_exp);
   for (int d = 0; d < 3; ++d)
     cudaFree(h->d_face_geo64[d]);
   for (int d = 0; d < 3; ++d)

@@ -12,6 +12,7 @@
 // (steps x stages launches + one step-advance launch per step) stays valid
 // while solves join and leave the batch.
 #include "batch_kernels.h"
+#include "stage_fx.cuh"
 #include "stage_gauss.cuh"
 
 namespace adv
@@ -23,7 +24,7 @@ constexpr bool kBatchCollocation = sizeof(T) == sizeof(double);
 
 // dynamic shared memory of the per-CTA code the group runs
 template <int N, typename T>
-constexpr int kBatchSmem = kBatchCollocation<T> ? GaussShape<N, T, true, false, true>::SMEM
+constexpr int kBatchSmem = kBatchCollocation<T> ? FxShape<N, true, true>::SMEM
                                                 : StageShape<N, T, true, false>::SMEM;
 
 template <int N, typename T>
@@ -55,6 +56,7 @@ __global__ void __launch_bounds__(StageShape<N, T, true, false>::THREADS) batch_
           a.periodic  = 7;
           a.uniform   = 1;
           a.out_scale = 1.0;
+          a.fx_ok     = S.fx_ok;
           // stage rotation of the three registers (as adv_lsrk_steps)
           const int  st   = L.stage;
           const bool last = st == L.n_stages - 1;
@@ -87,7 +89,12 @@ __global__ void __launch_bounds__(StageShape<N, T, true, false>::THREADS) batch_
   if (skip)
     return;
   if constexpr (kBatchCollocation<T>)
-    stage_gauss_cta<N, T, true, false, true>(sA, cell0, smem_raw);
+    {
+      if (sA.fx_ok)
+        stage_fx_cta<N, true, true, false, false>(sA, cell0, smem_raw);
+      else
+        stage_gauss_masked<N, true, true, false, false>(sA, cell0, smem_raw, ~0u);
+    }
   else
     stage_cta<N, T, true, false>(sA, cell0, smem_raw);
 }
@@ -117,7 +124,8 @@ cudaError_t launch_batch_t(const BatchLaunch &L, int cta_capacity, cudaStream_t 
 
 cudaError_t upload_tables_batch(const DevTables<double> *d, const DevTables<float> *f)
 {
-  return upload_tables_local(d, f);
+  cudaError_t e = upload_tables_local(d, f);
+  return e != cudaSuccess ? e : upload_fx_local(d);
 }
 
 bool batch_collocation(int precision)

@@ -19,7 +19,7 @@ struct BatchSlot
   double    dt;
   double    cv[3], P[3], M[3];    // uniform operator constants (a_d / h and the upwind split)
   float     cvf[3], Pf[3], Mf[3];
-  int       pad;
+  int       fx_ok; // cv within the block fixed-point window (in_fx_window)
 };
 
 struct BatchLaunch

@@ -1,0 +1,241 @@
+// Block fixed-point arithmetic for the contractions of the FP64 operator.
+//
+// On this GPU the FP64 pipe retires 2 instructions per clock and SM, the
+// integer multiply-add pipe about 55-64 32 x 32 -> 64 bit products (measured:
+// 1.6 DFMA, 53 mad.wide.s32, 61 shifts, 65 logic operations per clock and
+// SM), so a contraction carried as integers of 57 bits costs a fraction of
+// its binary64 form and is at least as exact: a block of values (a cell) is
+// scaled by one power of two above its largest entry and each value becomes
+//     X = x 2^(57 - E),  |X| <= 2^57,   X = h 2^29 + l,  |l| <= 2^28,
+// two signed 32-bit limbs (round to nearest).  A product with a constant of
+// the same form keeps h h', h l' + l h' in two 64-bit accumulators; the
+// dropped l l' is at most 2^-1 of the unit.  Rounding errors are thus a few
+// times 2^-57 of the block's largest entry per contraction, where binary64
+// commits 2^-53 of each intermediate result.
+//
+// Blocks whose scale leaves a safe window (infinities, NaN, values near the
+// ends of the binary64 range) are computed in binary64 by the caller.
+#pragma once
+
+#include "device_common.cuh"
+
+namespace adv
+{
+struct Limbs
+{
+  int h, l; // h 2^29 + l, |l| <= 2^28
+};
+
+__device__ __forceinline__ long long mad_wide(int a, int b, long long c)
+{
+  // inline PTX: the compiler splits the C expression into a product and a
+  // 64-bit addition, half the rate
+  asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(c) : "r"(a), "r"(b));
+  return c;
+}
+__device__ __forceinline__ long long mul_wide(int a, int b)
+{
+  return (long long)a * b;
+}
+
+// sum of products of limb pairs: value 2^58 hi + 2^29 mid
+struct FxAcc
+{
+  long long hi, mid;
+  // first product; `half` rounds the final shift of mid
+  __device__ __forceinline__ void set(int h, int l, int ch, int cl, long long half)
+  {
+    hi  = mul_wide(h, ch);
+    mid = mad_wide(l, ch, mad_wide(h, cl, half));
+  }
+  __device__ __forceinline__ void add(int h, int l, int ch, int cl)
+  {
+    hi  = mad_wide(h, ch, hi);
+    mid = mad_wide(h, cl, mid);
+    mid = mad_wide(l, ch, mid);
+  }
+};
+
+// Limbs of T / 2 rounded to nearest, |T| <= 2^58
+__device__ __forceinline__ Limbs fx_split(long long T)
+{
+  const long long Y = T + ((1ll << 29) + 1);
+  Limbs           r;
+  r.h = (int)(Y >> 30);
+  r.l = (int)(((unsigned)Y >> 1) & 0x1FFFFFFFu) - (1 << 28);
+  return r;
+}
+
+// biased binary64 exponent and magnitude bits of the high word
+__device__ __forceinline__ unsigned abs_hi(double x)
+{
+  return (unsigned)__double2hiint(x) & 0x7FFFFFFFu;
+}
+
+// x 2^(57 - E) as limbs for |x| < 2^E: top = E + 1022, the largest biased
+// exponent in the block
+__device__ __forceinline__ Limbs fx_from_double(double x, int top)
+{
+  const int      hi = __double2hiint(x);
+  const unsigned lo = (unsigned)__double2loint(x);
+  const int      s  = min(top - (int)(((unsigned)hi << 1) >> 21), 63);
+  const unsigned long long m = ((unsigned long long)(((unsigned)hi & 0xFFFFFu) | 0x100000u) << 32) | lo;
+  const int      sg = (hi >> 31) | 1;
+  Limbs          r  = fx_split((long long)((m << 5) >> s));
+  r.h *= sg;
+  r.l *= sg;
+  return r;
+}
+
+// X y 2^-Ey as limbs: the product of a fixed-point value with a binary64
+// factor |y| < 2^Ey (top = Ey + 1022), shifted down by the bits added to
+// top; y's mantissa, shifted to 57 bits, is the second limb pair
+__device__ __forceinline__ Limbs fx_times_double(Limbs X, double y, int top_plus_shift)
+{
+  const int      hi = __double2hiint(y);
+  const unsigned lo = (unsigned)__double2loint(y);
+  const int      s  = min(top_plus_shift - (int)(((unsigned)hi << 1) >> 21), 63);
+  const int      sg = (hi >> 31) | 1;
+  const int      mh = (int)__funnelshift_l(lo, ((unsigned)hi & 0xFFFFFu) | 0x100000u, 7) * sg;
+  const int      ml = (int)(lo & 0x1FFFFFFu) * (sg * 16);
+  FxAcc          p;
+  p.set(X.h, X.l, mh, ml, 0);
+  return fx_split(((p.hi << 2) + (p.mid >> 27)) >> s);
+}
+
+// X C 2^-57 shifted down by `shift`, C = (ch, cl) of the same form
+__device__ __forceinline__ Limbs fx_times(Limbs X, Limbs C, int shift)
+{
+  FxAcc p;
+  p.set(X.h, X.l, C.h, C.l, 0);
+  return fx_split(((p.hi << 2) + (p.mid >> 27)) >> shift);
+}
+
+// Z 2^e rounded to binary64, |Z| < 2^62, for normal results (on the integer
+// pipes: the conversion instruction issues on the FP64 pipe)
+__device__ __forceinline__ double fx_to_double(long long Z, int e)
+{
+  const unsigned long long s  = (unsigned long long)(Z >> 63);
+  const unsigned long long m  = ((unsigned long long)Z ^ s) - s;
+  const int                lz = __clzll((long long)m);
+  // leading bit to 62, round half up at bit 10; a carry moves the exponent on
+  const unsigned long long n = ((m << (lz - 1)) + 0x200u) >> 10;
+  const unsigned long long b = n + ((unsigned long long)(unsigned)(1023 + 62 - lz + e) << 52);
+  return __longlong_as_double((long long)(m ? (b | (s & 0x8000000000000000ull)) : 0ull));
+}
+
+// Constant tables.  The entries of the antisymmetric even-odd form of Dw
+// and of the face lifts are c 2^(57 - kd): 2^kd bounds the largest of them.
+// A product with a value X is kept at 2^(kFxGuard - kd) of X's unit, so
+// that the sum over three directions and six lifts of a cell stays below
+// 2^62: 3 (||Dw||_inf + max_q (|lw0| + |lw1|)) 2^(57 + kFxGuard - kd) is at
+// most 2^61.4 for n = 2..7 (20.8, 39.7, 64.0, 93.9, 129.4, 170.6 for the
+// bracket).
+constexpr int kFxGuard = 2;
+template <int N>
+constexpr int fx_kd()
+{
+  return N == 2 ? 2 : N == 3 ? 3 : N <= 5 ? 4 : 5;
+}
+
+struct FxEvenOdd
+{
+  int2 e[3][3], o[3][3], ce[3], mid[3];
+};
+
+struct FxTables
+{
+  FxEvenOdd Dw;
+  int2      lwe[4], lwo[4];
+};
+
+static __constant__ FxTables c_tab_fx[kMaxNDev + 1];
+
+// c 2^bits as balanced limbs
+inline int2 fx_host_limbs(double c, int bits)
+{
+  const long long X = llrint(ldexp(c, bits));
+  const long long l = ((X + (1ll << 28)) & ((1ll << 29) - 1)) - (1ll << 28);
+  return make_int2((int)((X - l) >> 29), (int)l);
+}
+
+inline cudaError_t upload_fx_local(const DevTables<double> *d)
+{
+  static FxTables t[kMaxNDev + 1];
+  memset(t, 0, sizeof(t));
+  const int kd[kMaxNDev + 1] = {0, 0, fx_kd<2>(), fx_kd<3>(), fx_kd<4>(), fx_kd<5>(), fx_kd<6>(), fx_kd<7>()};
+  for (int n = 2; n <= kMaxNDev; ++n)
+    {
+      const EvenOdd<double> &M    = d[n].Dw_eo;
+      const int              bits = 57 - kd[n], h = n / 2;
+      for (int q = 0; q < h; ++q)
+        {
+          for (int i = 0; i < h; ++i)
+            {
+              t[n].Dw.e[q][i] = fx_host_limbs(M.e[q][i], bits);
+              t[n].Dw.o[q][i] = fx_host_limbs(M.o[q][i], bits);
+            }
+          t[n].Dw.ce[q]  = fx_host_limbs(M.ce[q], bits);
+          t[n].Dw.mid[q] = fx_host_limbs(M.mid[q], bits);
+          t[n].lwo[q]    = fx_host_limbs(d[n].lwo[q], bits);
+        }
+      for (int q = 0; q < (n + 1) / 2; ++q)
+        t[n].lwe[q] = fx_host_limbs(d[n].lwe[q], bits);
+    }
+  return cudaMemcpyToSymbol(c_tab_fx, t, sizeof(t));
+}
+
+// Fixed-point value of an accumulator of products with table constants,
+// rounded to nearest (started with kFxHalf): a truncation's bias would be the
+// same in every stage and add up over the steps
+constexpr long long kFxHalf = 1ll << (27 - kFxGuard);
+__device__ __forceinline__ long long fx_value(const FxAcc &a)
+{
+  return (a.hi << (1 + kFxGuard)) + (a.mid >> (28 - kFxGuard));
+}
+
+// Volume and lift terms of one pencil: out = Dw V + lw0 F_lo + lw1 F_hi from
+// the even-odd halves, in units of 2^(kFxGuard - kd) of V's and F's
+template <int N>
+__device__ __forceinline__ void fx_sweep_lift(const FxTables &tb, const Limbs (&V)[N], Limbs Flo, Limbs Fhi,
+                                              long long (&out)[N])
+{
+  constexpr int H   = N / 2;
+  const int     psh = Flo.h + Fhi.h, psl = Flo.l + Fhi.l;
+  const int     pdh = Flo.h - Fhi.h, pdl = Flo.l - Fhi.l;
+  int           eh[H], el[H], oh[H], ol[H];
+#pragma unroll
+  for (int i = 0; i < H; ++i)
+    {
+      eh[i] = V[i].h + V[N - 1 - i].h, el[i] = V[i].l + V[N - 1 - i].l;
+      oh[i] = V[i].h - V[N - 1 - i].h, ol[i] = V[i].l - V[N - 1 - i].l;
+    }
+#pragma unroll
+  for (int q = 0; q < H; ++q)
+    {
+      FxAcc E, O;
+      O.set(psh, psl, tb.lwe[q].x, tb.lwe[q].y, kFxHalf);
+      E.set(pdh, pdl, tb.lwo[q].x, tb.lwo[q].y, kFxHalf);
+#pragma unroll
+      for (int i = 0; i < H; ++i)
+        {
+          E.add(eh[i], el[i], tb.Dw.e[q][i].x, tb.Dw.e[q][i].y);
+          O.add(oh[i], ol[i], tb.Dw.o[q][i].x, tb.Dw.o[q][i].y);
+        }
+      if (N % 2)
+        E.add(V[H].h, V[H].l, tb.Dw.ce[q].x, tb.Dw.ce[q].y);
+      const long long a = fx_value(O), b = fx_value(E);
+      out[q]         = a + b;
+      out[N - 1 - q] = a - b;
+    }
+  if (N % 2)
+    {
+      FxAcc m;
+      m.set(psh, psl, tb.lwe[H].x, tb.lwe[H].y, kFxHalf);
+#pragma unroll
+      for (int i = 0; i < H; ++i)
+        m.add(oh[i], ol[i], tb.Dw.mid[i].x, tb.Dw.mid[i].y);
+      out[H] = fx_value(m);
+    }
+}
+} // namespace adv

@@ -222,6 +222,11 @@ int setup_slab(const adv_config &cfg, int z_begin, int z_end, Mesh &m)
   return 0;
 }
 
+bool in_fx_window(double x)
+{
+  return std::fabs(x) > 0x1p-200 && std::fabs(x) < 0x1p200;
+}
+
 void compute_geometry(const adv_config &cfg, const Mesh &m, const Tables1D &tb, HostGeometry &g)
 {
   const int    n = m.n, nq = n * n * n, nf = n * n;
@@ -274,15 +279,18 @@ void compute_geometry(const adv_config &cfg, const Mesh &m, const Tables1D &tb, 
           g.P[d]  = 0.5 * (g.cv[d] + alpha * std::fabs(g.cv[d]));
           g.M[d]  = 0.5 * (g.cv[d] - alpha * std::fabs(g.cv[d]));
         }
+      g.fx_ok = in_fx_window(std::max({std::fabs(g.cv[0]), std::fabs(g.cv[1]), std::fabs(g.cv[2])}));
     }
   else
     {
       g.cell.assign((size_t)m.n_cells * 4 * nq, 0.0);
+      g.cell_exp.assign((size_t)m.n_cells, 0);
+      int outside = 0;
       double S[kMaxN * kMaxN], Sd[kMaxN * kMaxN];
       for (int q = 0; q < n; ++q)
         for (int i = 0; i < n; ++i)
           S[q * n + i] = tb.S[q][i], Sd[q * n + i] = tb.Sd[q][i];
-#pragma omp parallel
+#pragma omp parallel reduction(| : outside)
       {
         std::vector<double> X(3 * nq), x(3 * nq), J(9 * nq);
 #pragma omp for schedule(static)
@@ -291,7 +299,7 @@ void compute_geometry(const adv_config &cfg, const Mesh &m, const Tables1D &tb, 
             cell_support_points(cfg, m, tb, c, X.data());
             map_grid_rel(n, X.data(), n, S, Sd, n, S, Sd, n, S, Sd, x.data(), J.data());
             double *out = &g.cell[(size_t)c * 4 * nq];
-            double  vavg[3] = {0.0, 0.0, 0.0}, vol = 0.0;
+            double  vavg[3] = {0.0, 0.0, 0.0}, vol = 0.0, vmax = 0.0;
             for (int q = 0; q < nq; ++q)
               {
                 double       Ji[9], b[3];
@@ -302,15 +310,21 @@ void compute_geometry(const adv_config &cfg, const Mesh &m, const Tables1D &tb, 
                   {
                     out[d * nq + q] = det * (Ji[3 * d + 0] * b[0] + Ji[3 * d + 1] * b[1] + Ji[3 * d + 2] * b[2]);
                     vavg[d] += out[d * nq + q] * w;
+                    vmax = std::max(vmax, std::fabs(out[d * nq + q]));
                   }
                 out[3 * nq + q] = 1.0 / det;
+                outside |= !in_fx_window(out[3 * nq + q]);
                 vol += det * w;
               }
+            // (a cell without velocity: any exponent in the window does)
+            outside |= vmax != 0.0 && !in_fx_window(vmax);
+            g.cell_exp[c] = vmax != 0.0 ? std::ilogb(vmax) + 1023 : 1023;
             for (int d = 0; d < 3; ++d)
               g.fdm_cell[4 * c + d] = vavg[d] / vol;
             g.fdm_cell[4 * c + 3] = 1.0 / vol;
           }
       }
+      g.fx_ok = !outside;
     }
 
   // faces: coefficients (field case) and Dirichlet point positions

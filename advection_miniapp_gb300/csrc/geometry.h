@@ -62,6 +62,12 @@ struct HostGeometry
   // Dirichlet: per direction, per face, n^2 points x 3 coordinates (boundary faces only hold data)
   std::vector<double> face_x[3];
   double h_min = 0.0;
+  // block fixed-point path: whether the metric is inside its window of
+  // exponents (uniform: the largest |cv|; field: vt's largest entry of every
+  // cell and every 1 / det J within 2^+-200), and in the field case the biased
+  // binary64 exponent of the largest |vt| of every cell
+  bool             fx_ok = false;
+  std::vector<int> cell_exp;
   // per cell (v0, v1, v2, 1/|K|): JxW-weighted cell average of J^{-1} b and the
   // inverse cell volume (the cell data of the FDM preconditioner,
   // advection_solver_implicit.cc:1063-1076)
@@ -80,5 +86,7 @@ void support_points(const adv_config &cfg, const Mesh &m, const Tables1D &tb, in
 int  setup_mesh(const adv_config &cfg, Mesh &m);
 // local mesh of the slab of global z layers [z_begin, z_end) with its ghost layers
 int  setup_slab(const adv_config &cfg, int z_begin, int z_end, Mesh &m);
+// magnitude within 2^-200 .. 2^200: metric factors the block fixed-point path takes
+bool in_fx_window(double x);
 void compute_geometry(const adv_config &cfg, const Mesh &m, const Tables1D &tb, HostGeometry &g);
 } // namespace adv

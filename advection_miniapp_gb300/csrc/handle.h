@@ -27,6 +27,8 @@ struct adv_handle
   void    *d_face_geo[3] = {};
   double  *d_cell_geo64    = nullptr;   // FP32 increments: the FP64 copy for the anchor stage
   double  *d_face_geo64[3] = {};
+  int     *d_cell_exp    = nullptr;     // field geometry: exponent of the largest |vt| per cell
+  bool     fx_ok         = false;       // the metric is inside the block fixed-point window
   double  *d_face_x[3]   = {};
   double  *d_partials    = nullptr;
   double  *d_scratch[2]  = {};

@@ -57,6 +57,11 @@ struct StageArgs
   float         mass_factorf;
   float         volf;        // uniform case: cell volume (det J)
   double        vol;
+  // block fixed-point path (stage_fx.cuh): allowed for this mesh (vt, 1 / det J
+  // or the uniform constants within 2^+-200), and in the field case the
+  // largest biased binary64 exponent of vt per cell
+  int           fx_ok;
+  const int    *cell_exp;
   const void   *cell_geo;    // field case: [vt0|vt1|vt2|idet] x n^3 per cell (T)
   const void   *face_geo[3]; // field case: n^2 (P, M) pairs per face (T)
   const double *face_x[3];   // Dirichlet faces: n^2 x 3 coordinates per face
@@ -103,6 +108,13 @@ cudaError_t launch_stage(int n, int precision, const StageArgs &args, cudaStream
 // coefficients on the Gauss-point basis, JxW (c u - L u) at each point.
 cudaError_t launch_stage_gauss_fp64(int n, const StageArgs &args, cudaStream_t stream);
 cudaError_t launch_stage_gauss_fp32(int n, const StageArgs &args, cudaStream_t stream);
+// the block fixed-point kernels (stage_fx.cuh) of 2-3, 4-5 and 6-7 points
+cudaError_t launch_stage_fx_a(int n, const StageArgs &args, cudaStream_t stream);
+cudaError_t launch_stage_fx_b(int n, const StageArgs &args, cudaStream_t stream);
+cudaError_t launch_stage_fx_c(int n, const StageArgs &args, cudaStream_t stream);
+cudaError_t upload_tables_fx_a(const DevTables<double> *d, const DevTables<float> *f);
+cudaError_t upload_tables_fx_b(const DevTables<double> *d, const DevTables<float> *f);
+cudaError_t upload_tables_fx_c(const DevTables<double> *d, const DevTables<float> *f);
 cudaError_t upload_tables_gauss64(const DevTables<double> *d, const DevTables<float> *f);
 cudaError_t upload_tables_gauss32(const DevTables<double> *d, const DevTables<float> *f);
 // In-place change of basis of the cells [cell_begin, cell_end) of u:

@@ -208,6 +208,7 @@ int rebuild(adv_server *S, SGroup &g)
           b.cv[d] = q.cv[d], b.P[d] = q.P[d], b.M[d] = q.M[d];
           b.cvf[d] = (float)q.cv[d], b.Pf[d] = (float)q.P[d], b.Mf[d] = (float)q.M[d];
         }
+      b.fx_ok = adv::in_fx_window(std::max({std::fabs(q.cv[0]), std::fabs(q.cv[1]), std::fabs(q.cv[2])}));
       const long long cells = (long long)q.n * q.n * q.n;
       for (long long c = 0; c < cells; c += C)
         {

@@ -1,0 +1,22 @@
+// Instantiations of the block fixed-point stage kernel: 4 and 5 points per
+// direction (split over translation units to compile in parallel).
+#include "stage_fx.cuh"
+
+namespace adv
+{
+cudaError_t upload_tables_fx_b(const DevTables<double> *d, const DevTables<float> *f)
+{
+  cudaError_t e = upload_tables_local(d, f);
+  return e != cudaSuccess ? e : upload_fx_local(d);
+}
+
+cudaError_t launch_stage_fx_b(int n, const StageArgs &args, cudaStream_t stream)
+{
+  switch (n)
+    {
+      case 4: return launch_stage_fx_n<4>(args, stream);
+      case 5: return launch_stage_fx_n<5>(args, stream);
+      default: return cudaErrorInvalidValue;
+    }
+}
+} // namespace adv

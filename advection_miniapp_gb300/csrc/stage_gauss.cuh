@@ -130,9 +130,10 @@ __device__ __forceinline__ bool upwind_pencil_traces(const DevTables<T> &tb, con
 // Binary32 operator: the input comes from r_in32 and the update is the
 // increment form's.  FP64 operator: the block's anchor (writes K0 and the
 // first G).
+// cell_mask: the cells of the CTA (bit cl) whose outputs are written.
 template <int N, typename T, bool UNI, bool VISC, bool TR = false, bool INC = false, bool UPW = false>
 __device__ __forceinline__ void stage_gauss_cta(const StageArgs &A, const long long cell0,
-                                                unsigned char *smem_raw)
+                                                unsigned char *smem_raw, unsigned cell_mask = ~0u)
 {
   using SH         = StageShape<N, T, UNI, VISC>;
   constexpr int C  = SH::C;
@@ -466,6 +467,8 @@ __device__ __forceinline__ void stage_gauss_cta(const StageArgs &A, const long l
   for (int w = tid; w < ncell * NF; w += NT)
     {
       const int cl = w / NF, r = w % NF;
+      if (!((cell_mask >> cl) & 1u))
+        continue;
       const T  *p  = Ub + cl * NQ + r;
       T         U[N], out[N];
 #pragma unroll
@@ -609,6 +612,8 @@ __device__ __forceinline__ void stage_gauss_cta(const StageArgs &A, const long l
         {
           const int dd = w / (ncell * NF), v = w % (ncell * NF);
           const int cl = v / NF, r = v % NF;
+          if (!((cell_mask >> cl) & 1u))
+            continue;
           const int off = dd == 0 ? N * r : (r % N) + NF * (r / N);
           const int st  = dd == 0 ? 1 : N;
           const T  *p   = Qb + cl * NQ + off;

@@ -164,6 +164,12 @@ cudaError_t upload_tables_gauss64(const DevTables<double> *d, const DevTables<fl
 
 cudaError_t launch_stage_gauss_fp64(int n, const StageArgs &args, cudaStream_t stream)
 {
+  // block fixed-point contractions wherever they apply: advection without a
+  // skew term, metric within the window of exponents
+  if (args.fx_ok && !args.visc && !args.has_skew)
+    return n <= 3 ? launch_stage_fx_a(n, args, stream)
+         : n <= 5 ? launch_stage_fx_b(n, args, stream)
+                  : launch_stage_fx_c(n, args, stream);
   return launch_stage_gauss_any<double>(n, args, stream);
 }
 

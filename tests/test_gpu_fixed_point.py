@@ -1,0 +1,94 @@
+"""Block fixed-point stages of the FP64 operator (collocation form) against the oracle.
+
+The scale of a cell's block adapts to its data, so a step commutes with any
+power of two, cells of very different magnitude sit side by side, and cells
+outside the window of exponents (here 2^-400 .. 2^600, infinities, NaN) take
+the binary64 path.  Bars: the repository's FP64 bar, 1e-12 of the largest
+entry; the fixed-point error is a few 2^-57 of a cell's largest intermediate
+value per contraction, below binary64's own rounding.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-12
+
+# uniform, curved with upwind traces, curved reading every trace, boundary data
+MESHES = {
+    "uniform": dict(n_cells=(3, 2, 5)),
+    "curved": dict(n_cells=(3, 3, 2), mesh_type=1, deformation=0.07),
+    "curved-lax-friedrichs": dict(n_cells=(2, 3, 3), mesh_type=1, deformation=0.06, flux_alpha=0.5),
+    "curved-dirichlet": dict(n_cells=(2, 3, 2), mesh_type=1, deformation=0.06, periodic=0, initial_condition=2),
+    "rotating": dict(n_cells=(2, 2, 3), periodic=0, velocity_type=1, velocity=(1.0, 1.0, 0.3), velocity_period=0.5,
+                     initial_condition=1, ic_params=(0.3, 0.5, 0.5, 0.1), boundary_value=0),
+}
+
+
+def gpu_step(torch, adv, cfg, u0, t, dt, steps=1, scheme=None, **kw):
+    op = adv.AdvectionOperation(**cfg, **kw)
+    u = torch.from_numpy(np.ascontiguousarray(u0)).cuda()
+    r, k = op.initialize_dof_vector(), op.initialize_dof_vector()
+    op.lsrk_steps(adv.LSRK_5_4 if scheme is None else scheme, t, dt, steps, u, r, k)
+    return u.cpu().numpy()
+
+
+def oracle_step(oracle_mod, cfg, u0, t, dt):
+    o = oracle_mod.Oracle(**cfg)
+    u, r, k = u0.copy(), np.zeros_like(u0), np.zeros_like(u0)
+    o.lsrk_step(t, dt, u, r, k)
+    return u
+
+
+@pytest.mark.parametrize("degree", [1, 2, 3, 4, 5, 6])
+@pytest.mark.parametrize("mesh", sorted(MESHES))
+def test_step_matches_oracle(cuda, oracle_mod, adv_lib, mesh, degree):
+    cfg = dict(MESHES[mesh], degree=degree)
+    u0 = np.random.default_rng(degree).standard_normal(oracle_mod.Oracle(**cfg).n_dofs)
+    ref = oracle_step(oracle_mod, cfg, u0, 0.1, 0.004)
+    for form in (adv_lib.FORM_AUTO, adv_lib.FORM_COLLOCATION_NO_TRACES):
+        got = gpu_step(cuda, adv_lib, cfg, u0, 0.1, 0.004, fused_form=form)
+        assert np.abs(got - ref).max() <= TOL * np.abs(ref).max(), (mesh, degree, form)
+
+
+# inside the window, at its lower and upper side, and outside both ends
+@pytest.mark.parametrize("exponent", [-900, -450, -300, 300, 620, 900])
+@pytest.mark.parametrize("mesh", ["uniform", "curved"])
+def test_step_commutes_with_powers_of_two(cuda, oracle_mod, adv_lib, mesh, exponent):
+    cfg = dict(MESHES[mesh], degree=3)
+    u0 = np.random.default_rng(3).standard_normal(oracle_mod.Oracle(**cfg).n_dofs)
+    ref = oracle_step(oracle_mod, cfg, u0, 0.0, 0.004)
+    got = np.ldexp(gpu_step(cuda, adv_lib, cfg, np.ldexp(u0, exponent), 0.0, 0.004), -exponent)
+    assert np.abs(got - ref).max() <= TOL * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("mesh", ["uniform", "curved"])
+def test_cells_of_different_magnitude(cuda, oracle_mod, adv_lib, mesh):
+    """Cells of 2^-470 and of 0 beside cells of 1: a large neighbour's flux
+    sets the scale of a small cell, and a cell alone in a small neighbourhood
+    takes the binary64 path."""
+    cfg = dict(MESHES[mesh], degree=4, n_cells=(6, 5, 4))
+    o = oracle_mod.Oracle(**cfg)
+    rng = np.random.default_rng(5)
+    u0 = rng.standard_normal(o.n_dofs).reshape(-1, 125)
+    u0[::7] = 0.0
+    u0[40:100] *= 2.0 ** -470
+    u0 = u0.reshape(-1)
+    ref = oracle_step(oracle_mod, cfg, u0, 0.0, 0.002)
+    got = gpu_step(cuda, adv_lib, cfg, u0, 0.0, 0.002)
+    assert np.abs(got - ref).max() <= TOL * np.abs(ref).max()
+    assert np.abs(got - gpu_step(cuda, adv_lib, cfg, u0, 0.0, 0.002,
+                                 fused_form=adv_lib.FORM_COLLOCATION_NO_TRACES)).max() == 0.0
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_values_that_are_not_finite_stay_local(cuda, oracle_mod, adv_lib, value):
+    cfg = dict(MESHES["curved"], degree=4, n_cells=(9, 4, 4))
+    n = oracle_mod.Oracle(**cfg).n_dofs
+    u0 = np.random.default_rng(6).standard_normal(n)
+    clean = gpu_step(cuda, adv_lib, cfg, u0, 0.0, 0.002, scheme=adv_lib.LSRK_3_3).reshape(4, 4, 9, 125)
+    u0[(2 + 9 * (1 + 4 * 1)) * 125 + 62] = value
+    got = gpu_step(cuda, adv_lib, cfg, u0, 0.0, 0.002, scheme=adv_lib.LSRK_3_3).reshape(4, 4, 9, 125)
+    assert not np.isfinite(got[1, 1, 2]).any()
+    # three stages reach at most three cells
+    np.testing.assert_array_equal(got[:, :, 6:8], clean[:, :, 6:8])
