@@ -54,18 +54,18 @@ struct DevTables
   T lde[kMaxNDev], ldo[kMaxNDev];
 };
 
-// Index [n] holds the tables of n points per direction.  The library is
+// Index [n - 2] holds the tables of n points per direction.  The library is
 // built without relocatable device code, so every translation unit that
 // includes this header owns a copy, filled by its own upload function.
-static __constant__ DevTables<double> c_tab_d[kMaxNDev + 1];
-static __constant__ DevTables<float>  c_tab_f[kMaxNDev + 1];
+static __constant__ DevTables<double> c_tab_d[kMaxNDev - 1];
+static __constant__ DevTables<float>  c_tab_f[kMaxNDev - 1];
 
 static inline cudaError_t upload_tables_local(const DevTables<double> *d, const DevTables<float> *f)
 {
-  cudaError_t e = cudaMemcpyToSymbol(c_tab_d, d, sizeof(c_tab_d));
+  cudaError_t e = cudaMemcpyToSymbol(c_tab_d, d + 2, sizeof(c_tab_d));
   if (e != cudaSuccess)
     return e;
-  return cudaMemcpyToSymbol(c_tab_f, f, sizeof(c_tab_f));
+  return cudaMemcpyToSymbol(c_tab_f, f + 2, sizeof(c_tab_f));
 }
 
 // One-time opt-in of a kernel's dynamic shared-memory size on the current
@@ -93,12 +93,12 @@ __device__ __forceinline__ const DevTables<T> &tab(int n);
 template <>
 __device__ __forceinline__ const DevTables<double> &tab<double>(int n)
 {
-  return c_tab_d[n];
+  return c_tab_d[n - 2];
 }
 template <>
 __device__ __forceinline__ const DevTables<float> &tab<float>(int n)
 {
-  return c_tab_f[n];
+  return c_tab_f[n - 2];
 }
 
 // binary64 -> binary32 by integer arithmetic (round half away from zero in

@@ -112,6 +112,9 @@ cudaError_t launch_stage_gauss_fp32(int n, const StageArgs &args, cudaStream_t s
 cudaError_t launch_stage_fx_a(int n, const StageArgs &args, cudaStream_t stream);
 cudaError_t launch_stage_fx_b(int n, const StageArgs &args, cudaStream_t stream);
 cudaError_t launch_stage_fx_c(int n, const StageArgs &args, cudaStream_t stream);
+cudaError_t launch_stage_fx_nodal_a(int n, const StageArgs &args, cudaStream_t stream);
+cudaError_t launch_stage_fx_nodal_b(int n, const StageArgs &args, cudaStream_t stream);
+cudaError_t launch_stage_fx_nodal_c(int n, const StageArgs &args, cudaStream_t stream);
 cudaError_t upload_tables_fx_a(const DevTables<double> *d, const DevTables<float> *f);
 cudaError_t upload_tables_fx_b(const DevTables<double> *d, const DevTables<float> *f);
 cudaError_t upload_tables_fx_c(const DevTables<double> *d, const DevTables<float> *f);

@@ -10,6 +10,11 @@ cudaError_t upload_tables_stage64(const DevTables<double> *d, const DevTables<fl
 
 cudaError_t launch_stage_fp64(int n, const StageArgs &args, cudaStream_t stream)
 {
+  // block fixed-point contractions wherever they apply (as launch_stage_gauss_fp64)
+  if (args.fx_ok && !args.visc && !args.has_skew)
+    return n <= 3 ? launch_stage_fx_nodal_a(n, args, stream)
+         : n <= 5 ? launch_stage_fx_nodal_b(n, args, stream)
+                  : launch_stage_fx_nodal_c(n, args, stream);
   switch (n)
     {
       case 2: return launch_stage_n<2, double>(args, stream);

@@ -47,23 +47,6 @@ struct FxShape
   static_assert(2 * C * N * N * N * 8 % 16 == 0, "cp.async destinations need 16-byte alignment");
 };
 
-// Neighbour cell (-1: boundary) and face id of face j of the cell at (ix, iy, iz)
-__device__ __forceinline__ void cell_face(const StageArgs &A, int ix, int iy, int iz, int j, int &nb, unsigned &face)
-{
-  const int  d = j >> 1, s = j & 1;
-  const int  nx = A.nc[0], ny = A.nc[1];
-  const int  id = d == 0 ? ix : d == 1 ? iy : iz, nd = A.nc[d];
-  const int  j1 = d == 0 ? iy : ix, j2 = d == 2 ? iy : iz, n1 = d == 0 ? ny : nx;
-  const bool wrap = (A.periodic >> d) & 1;
-  const int  pos = wrap && id + s == nd ? 0 : id + s;
-  face           = (unsigned)pos + (unsigned)A.npos[d] * ((unsigned)j1 + (unsigned)n1 * (unsigned)j2);
-  int q          = id + 2 * s - 1;
-  if (wrap)
-    q = q < 0 ? nd - 1 : q == nd ? 0 : q;
-  const int jx = d == 0 ? q : ix, jy = d == 1 ? q : iy, jz = d == 2 ? q : iz;
-  nb           = q < 0 || q >= nd ? -1 : jx + nx * (jy + ny * jz);
-}
-
 // the binary64 path for the cells of `mask`
 template <int N, bool UNI, bool TR, bool INC, bool UPW>
 __device__ __noinline__ void stage_gauss_masked(const StageArgs &A, long long cell0, unsigned char *smem,
@@ -450,12 +433,6 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
       stage_gauss_masked<N, UNI, TR, INC, UPW>(A, cell0, smem_raw, bad);
     }
 }
-
-// resident threads per SM the register allocation allows for (80 registers a
-// thread); measured on 64^3 curved cells of degree 4, 4 steps: 16.61 ms with
-// 768, 16.67 with 640, 16.54 with 896, 18.72 with 512; 29 x 23 x 37 affine
-// cells of degree 2: 686, 730, 682 and 733 us
-constexpr int kFxThreadsPerSM = 768;
 
 template <int N, bool UNI, bool TR, bool INC, bool UPW>
 __global__ void __launch_bounds__(FxShape<N, UNI, TR>::THREADS, kFxThreadsPerSM / FxShape<N, UNI, TR>::THREADS)

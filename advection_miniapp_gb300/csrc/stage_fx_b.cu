@@ -1,13 +1,16 @@
-// Instantiations of the block fixed-point stage kernel: 4 and 5 points per
+// Instantiations of the block fixed-point stage kernels: 4 and 5 points per
 // direction (split over translation units to compile in parallel).
 #include "stage_fx.cuh"
+#include "stage_fx_nodal.cuh"
 
 namespace adv
 {
 cudaError_t upload_tables_fx_b(const DevTables<double> *d, const DevTables<float> *f)
 {
   cudaError_t e = upload_tables_local(d, f);
-  return e != cudaSuccess ? e : upload_fx_local(d);
+  if (e == cudaSuccess)
+    e = upload_fx_local(d);
+  return e != cudaSuccess ? e : upload_fx_basis_local(d);
 }
 
 cudaError_t launch_stage_fx_b(int n, const StageArgs &args, cudaStream_t stream)
@@ -16,6 +19,16 @@ cudaError_t launch_stage_fx_b(int n, const StageArgs &args, cudaStream_t stream)
     {
       case 4: return launch_stage_fx_n<4>(args, stream);
       case 5: return launch_stage_fx_n<5>(args, stream);
+      default: return cudaErrorInvalidValue;
+    }
+}
+
+cudaError_t launch_stage_fx_nodal_b(int n, const StageArgs &args, cudaStream_t stream)
+{
+  switch (n)
+    {
+      case 4: return launch_stage_fx_nodal_n<4>(args, stream);
+      case 5: return launch_stage_fx_nodal_n<5>(args, stream);
       default: return cudaErrorInvalidValue;
     }
 }

@@ -540,6 +540,23 @@ __device__ __forceinline__ void cell_neighbours(const StageArgs &A, long long ce
     }
 }
 
+// Neighbour cell (-1: boundary) and face id of face j of the cell at (ix, iy, iz)
+__device__ __forceinline__ void cell_face(const StageArgs &A, int ix, int iy, int iz, int j, int &nb, unsigned &face)
+{
+  const int  d = j >> 1, s = j & 1;
+  const int  nx = A.nc[0], ny = A.nc[1];
+  const int  id = d == 0 ? ix : d == 1 ? iy : iz, nd = A.nc[d];
+  const int  j1 = d == 0 ? iy : ix, j2 = d == 2 ? iy : iz, n1 = d == 0 ? ny : nx;
+  const bool wrap = (A.periodic >> d) & 1;
+  const int  pos = wrap && id + s == nd ? 0 : id + s;
+  face           = (unsigned)pos + (unsigned)A.npos[d] * ((unsigned)j1 + (unsigned)n1 * (unsigned)j2);
+  int q          = id + 2 * s - 1;
+  if (wrap)
+    q = q < 0 ? nd - 1 : q == nd ? 0 : q;
+  const int jx = d == 0 ? q : ix, jy = d == 1 ? q : iy, jz = d == 2 ? q : iz;
+  nb           = q < 0 || q >= nd ? -1 : jx + nx * (jy + ny * jz);
+}
+
 // Field case: asynchronous copies of the cell geometry (16-byte chunks) and
 // the face coefficients (8-byte chunks) into shared memory, committed as one
 // group; the caller waits with __pipeline_wait_prior(0) before using them.
@@ -570,7 +587,8 @@ __device__ __forceinline__ void geometry_async(const StageArgs &A, long long cel
 // with the dynamic shared memory of the launch.  Shared by the single-mesh
 // kernel and the batched multi-mesh kernel of the serving loop.
 template <int N, typename T, bool UNI, bool VISC>
-__device__ __forceinline__ void stage_cta(const StageArgs &A, const long long cell0, unsigned char *smem_raw)
+__device__ __forceinline__ void stage_cta(const StageArgs &A, const long long cell0, unsigned char *smem_raw,
+                                          unsigned cell_mask = ~0u)
 {
   using SH         = StageShape<N, T, UNI, VISC>;
   constexpr int C  = SH::C;
@@ -893,21 +911,27 @@ __device__ __forceinline__ void stage_cta(const StageArgs &A, const long long ce
 
   // ---- phase 8: Runge-Kutta update over the CTA's contiguous DoF range
   //      (the post-operation lambda of advection_solver.cc:728-752)
-  const long long g0 = cell0 * NQ;
+  //      of the cells of cell_mask
+  const long long g0     = cell0 * NQ;
+  auto            masked = [&](int i) { return cell_mask != ~0u && !((cell_mask >> (i / NQ)) & 1u); };
   if (A.mode == kModeVmult)
     {
       for (int i = tid; i < ncell * NQ; i += NT)
-        A.r_out[g0 + i] = to_double<T>(Qb[i]);
+        if (!masked(i))
+          A.r_out[g0 + i] = to_double<T>(Qb[i]);
     }
   else if (A.mode == kModeApply)
     {
       for (int i = tid; i < ncell * NQ; i += NT)
-        A.r_out[g0 + i] = A.out_scale * to_double<T>(Qb[i]);
+        if (!masked(i))
+          A.r_out[g0 + i] = A.out_scale * to_double<T>(Qb[i]);
     }
   else if (A.mode == kModeStage)
     {
       for (int i = tid; i < ncell * NQ; i += NT)
         {
+          if (masked(i))
+            continue;
           double kd = to_double<T>(Qb[i]);
           if (A.k_add)
             kd += __ldcs(A.k_add + g0 + i);
@@ -922,6 +946,8 @@ __device__ __forceinline__ void stage_cta(const StageArgs &A, const long long ce
     {
       for (int i = tid; i < ncell * NQ; i += NT)
         {
+          if (masked(i))
+            continue;
           double kd = to_double<T>(Qb[i]);
           if (A.k_add)
             kd += __ldcs(A.k_add + g0 + i);

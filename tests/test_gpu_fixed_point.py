@@ -92,3 +92,77 @@ def test_values_that_are_not_finite_stay_local(cuda, oracle_mod, adv_lib, value)
     assert not np.isfinite(got[1, 1, 2]).any()
     # three stages reach at most three cells
     np.testing.assert_array_equal(got[:, :, 6:8], clean[:, :, 6:8])
+
+
+# ---- nodal kernel (apply, perform_stage, vmult)
+
+
+@pytest.mark.parametrize("degree", [1, 2, 3, 4, 5, 6])
+@pytest.mark.parametrize("mesh", sorted(MESHES))
+def test_apply_and_vmult_match_oracle(cuda, oracle_mod, adv_lib, mesh, degree):
+    cfg = dict(MESHES[mesh], degree=degree)
+    o, op = oracle_mod.Oracle(**cfg), adv_lib.AdvectionOperation(**cfg)
+    src = np.random.default_rng(20 + degree).standard_normal(o.n_dofs)
+    s, d = cuda.from_numpy(src).cuda(), op.initialize_dof_vector()
+    op.apply(s, d, 0.1)
+    ref = o.apply(src, 0.1)
+    assert np.abs(d.cpu().numpy() - ref).max() <= TOL * np.abs(ref).max()
+    # weak form: c M u - L u = M (c u - M^{-1} L u)
+    op.vmult(s, d, 3.0, 0.1)
+    e = op.initialize_dof_vector()
+    op.apply_mass(cuda.from_numpy(3.0 * src - ref).cuda(), e)
+    e = e.cpu().numpy()
+    assert np.abs(d.cpu().numpy() - e).max() <= TOL * np.abs(e).max()
+
+
+@pytest.mark.parametrize("exponent", [-900, -450, -300, 300, 620, 900])
+@pytest.mark.parametrize("mesh", ["uniform", "curved"])
+def test_apply_commutes_with_powers_of_two(cuda, oracle_mod, adv_lib, mesh, exponent):
+    cfg = dict(MESHES[mesh], degree=5)
+    o, op = oracle_mod.Oracle(**cfg), adv_lib.AdvectionOperation(**cfg)
+    src = np.random.default_rng(9).standard_normal(o.n_dofs)
+    s, d = cuda.from_numpy(np.ldexp(src, exponent)).cuda(), op.initialize_dof_vector()
+    op.apply(s, d, 0.0)
+    ref = o.apply(src, 0.0)
+    assert np.abs(np.ldexp(d.cpu().numpy(), -exponent) - ref).max() <= TOL * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("mesh", ["uniform", "curved"])
+def test_apply_on_cells_of_different_magnitude(cuda, oracle_mod, adv_lib, mesh):
+    cfg = dict(MESHES[mesh], degree=4, n_cells=(6, 5, 4))
+    o, op = oracle_mod.Oracle(**cfg), adv_lib.AdvectionOperation(**cfg)
+    src = np.random.default_rng(8).standard_normal(o.n_dofs).reshape(-1, 125)
+    src[::7] = 0.0
+    src[20:90] *= 2.0 ** -470  # some with neighbours of 1, some among their like
+    src = src.reshape(-1)
+    s, d = cuda.from_numpy(src).cuda(), op.initialize_dof_vector()
+    op.apply(s, d, 0.0)
+    ref, got = o.apply(src, 0.0), d.cpu().numpy()
+    assert np.abs(got - ref).max() <= TOL * np.abs(ref).max()
+    small = np.abs(ref).reshape(-1, 125).max(axis=1) < 2.0 ** -400  # cells that see no value of 1
+    small = np.repeat(small, 125)
+    assert small.any()
+    assert np.abs(got - ref)[small].max() <= TOL * np.abs(ref[small]).max()
+    # one value that is not finite reaches its own cell and the face neighbours
+    src[62 + 125 * 40] = np.nan
+    op.apply(cuda.from_numpy(src).cuda(), d, 0.0)
+    bad = ~np.isfinite(d.cpu().numpy()).reshape(-1, 125).all(axis=1)
+    assert bad[40] and bad.sum() <= 7
+    keep = np.repeat(~bad, 125)
+    np.testing.assert_array_equal(d.cpu().numpy()[keep], got[keep])
+
+
+def test_stage_in_place_outside_the_window(cuda, oracle_mod, adv_lib):
+    """The binary64 pass over single cells of a block reads the solution that
+    the block's other cells have already overwritten elsewhere."""
+    cfg = dict(MESHES["uniform"], degree=4, n_cells=(5, 4, 3))
+    o, op = oracle_mod.Oracle(**cfg), adv_lib.AdvectionOperation(**cfg)
+    rng = np.random.default_rng(10)
+    scale = np.where(np.arange(60) % 5 == 2, 2.0 ** -700, 1.0)[:, None]
+    u0, r0 = ((rng.standard_normal((60, 125)) * scale).reshape(-1) for _ in range(2))
+    uo, ro = u0.copy(), r0.copy()
+    o.perform_stage(0.0, 0.013, 0.021, ro, np.zeros_like(u0), uo, ro)
+    u, r, k = cuda.from_numpy(u0).cuda(), cuda.from_numpy(r0).cuda(), op.initialize_dof_vector()
+    op.perform_stage(0.0, 0.013, 0.021, r, k, u, r)
+    assert np.abs(u.cpu().numpy() - uo).max() <= TOL * np.abs(uo).max()
+    assert np.abs(r.cpu().numpy() - ro).max() <= TOL * np.abs(ro).max()
