@@ -235,6 +235,20 @@ int upload_array(const std::vector<double> &src, void **dst, int64_t &bytes)
   return ADV_OK;
 }
 
+// vt of the field geometry in the form the block fixed-point kernels read
+void vt_to_limbs(const adv::Mesh &m, adv::HostGeometry &g)
+{
+  const int64_t nq = (int64_t)m.n * m.n * m.n;
+#pragma omp parallel for schedule(static)
+  for (int64_t c = 0; c < m.n_cells; ++c)
+    for (int64_t i = 0; i < 3 * nq; ++i)
+      {
+        double    &v = g.cell[c * 4 * nq + i];
+        const int2 l = adv::fx_const58(v, g.cell_exp[c]);
+        std::memcpy(&v, &l, sizeof(v));
+      }
+}
+
 void fill_diag(adv_handle &h)
 {
   adv::detail::make_diag(h.cfg, h.mesh, h.tb, h.diag);
@@ -340,6 +354,7 @@ adv::StageArgs base_args(const adv_handle &h, double t, int prec = -1)
   A.cell_geo = geo64 ? (const void *)h.d_cell_geo64 : h.d_cell_geo;
   A.fx_ok    = h.fx_ok;
   A.cell_exp = h.d_cell_exp;
+  A.vt_limbs = h.fx_ok;
   A.t        = t;
   A.ex       = h.diag.ex;
   const double s = time_factor(h, t);
@@ -600,7 +615,7 @@ int create_handle(const adv_config *cfg, int z_begin, int z_end, adv_handle **ou
       const bool fp64 = h->cfg.precision == ADV_PRECISION_FP64;
       const bool both = h->cfg.precision == ADV_PRECISION_FP32_INCREMENT;
       // the block fixed-point stages: every form with an FP64 operator
-      h->fx_ok = g.fx_ok && (fp64 || both);
+      h->fx_ok = g.fx_ok && (fp64 || both) && h->cfg.diffusion == 0.0 && h->cfg.factor_skew == 0.0;
       if (h->fx_ok && !g.cell_exp.empty())
         {
           const size_t nb = g.cell_exp.size() * sizeof(int);
@@ -614,8 +629,12 @@ int create_handle(const adv_config *cfg, int z_begin, int z_end, adv_handle **ou
         }
       if (!g.cell.empty())
         {
+          if (fp64 && h->fx_ok)
+            vt_to_limbs(h->mesh, g);
           rc = fp64 ? upload_array<double>(g.cell, &h->d_cell_geo, h->device_bytes)
                     : upload_array<float>(g.cell, &h->d_cell_geo, h->device_bytes);
+          if (both && h->fx_ok)
+            vt_to_limbs(h->mesh, g);
           if (rc == ADV_OK && both)
             rc = upload_array<double>(g.cell, (void **)&h->d_cell_geo64, h->device_bytes);
         }

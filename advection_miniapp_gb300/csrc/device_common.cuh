@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include <atomic>
 
@@ -135,6 +136,27 @@ __device__ __forceinline__ double f2d_int(float f)
     hi = sign | 0x7FF00000u | ((a >> 3) & 0x000FFFFFu);
   const unsigned lo = zero ? 0u : (b << 29);
   return __hiloint2double((int)hi, (int)lo);
+}
+
+// Block fixed-point form (fixed.cuh) of a metric value:
+// y 2^(58 - Ey) as limbs h 2^29 + l (x = h, y = l, |l| <= 2^28) for |y| < 2^Ey (top = Ey + 1022): the form of the
+// uniform constants and of vt in the cell geometry
+__host__ __device__ __forceinline__ int2 fx_const58(double y, int top)
+{
+#ifdef __CUDA_ARCH__
+  const long long b = __double_as_longlong(y);
+#else
+  long long b;
+  memcpy(&b, &y, sizeof(b));
+#endif
+  const int       e = (int)((b >> 52) & 0x7FF); // (0 and subnormal values round to 0)
+  const int       s = top - e < 63 ? top - e : 63;
+  const long long m = (b & 0xFFFFFFFFFFFFFll) | (1ll << 52);
+  // |y| 2^(58 - Ey) = m 2^5 2^-s, rounded
+  long long v = s > 5 ? (m + (1ll << (s - 6))) >> (s - 5) : m << (5 - s);
+  v           = b < 0 ? -v : v;
+  const long long l = ((v + (1ll << 28)) & ((1ll << 29) - 1)) - (1ll << 28);
+  return make_int2((int)((v - l) >> 29), (int)l);
 }
 
 template <typename T>

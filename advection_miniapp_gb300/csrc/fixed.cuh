@@ -44,25 +44,36 @@ __device__ __forceinline__ long long mul_wide(int a, int b)
   return (long long)a * b;
 }
 
-// sum of products of limb pairs: value 2^58 hi + 2^29 mid
+// a constant's limbs h, l, and h shifted up by the bits between the high
+// accumulator and the result's unit
+struct FxConst
+{
+  int h, l, hs;
+};
+
+// Sum of products of limb pairs X with constants c 2^b, SHIFT the shift of
+// the constants' hs: hi + (mid >> (29 - SHIFT)) is X c 2^(b + SHIFT - 58),
+// rounded to nearest (mid starts at half a unit: a truncation's bias would be
+// the same in every stage and add up over the steps)
+template <int SHIFT>
 struct FxAcc
 {
   long long hi, mid;
-  // first product; `half` rounds the final shift of mid
-  __device__ __forceinline__ void set(int h, int l, int ch, int cl, long long half)
+  __device__ __forceinline__ void set(int h, int l, const FxConst &c)
   {
-    hi  = mul_wide(h, ch);
-    mid = mad_wide(l, ch, mad_wide(h, cl, half));
+    hi  = mul_wide(h, c.hs);
+    mid = mad_wide(l, c.h, mad_wide(h, c.l, 1ll << (28 - SHIFT)));
   }
-  __device__ __forceinline__ void add(int h, int l, int ch, int cl)
+  __device__ __forceinline__ void add(int h, int l, const FxConst &c)
   {
-    hi  = mad_wide(h, ch, hi);
-    mid = mad_wide(h, cl, mid);
-    mid = mad_wide(l, ch, mid);
+    hi  = mad_wide(h, c.hs, hi);
+    mid = mad_wide(h, c.l, mid);
+    mid = mad_wide(l, c.h, mid);
   }
+  __device__ __forceinline__ long long value() const { return hi + (mid >> (29 - SHIFT)); }
 };
 
-// Limbs of T / 2 rounded to nearest, |T| <= 2^58
+// Limbs of T / 2 rounded to nearest, |T| < 2^60
 __device__ __forceinline__ Limbs fx_split(long long T)
 {
   const long long Y = T + ((1ll << 29) + 1);
@@ -93,28 +104,46 @@ __device__ __forceinline__ Limbs fx_from_double(double x, int top)
   return r;
 }
 
-// X y 2^-Ey as limbs: the product of a fixed-point value with a binary64
-// factor |y| < 2^Ey (top = Ey + 1022), shifted down by the bits added to
-// top; y's mantissa, shifted to 57 bits, is the second limb pair
-__device__ __forceinline__ Limbs fx_times_double(Limbs X, double y, int top_plus_shift)
+// top exponent of the product c v (|c v| < 2^(top - 1022)); 0 for a product
+// with zero (v may then be a trace that nobody wrote), 2047 if v is not finite
+__device__ __forceinline__ unsigned fx_product_top(double c, double v)
 {
-  const int      hi = __double2hiint(y);
-  const unsigned lo = (unsigned)__double2loint(y);
-  const int      s  = min(top_plus_shift - (int)(((unsigned)hi << 1) >> 21), 63);
-  const int      sg = (hi >> 31) | 1;
-  const int      mh = (int)__funnelshift_l(lo, ((unsigned)hi & 0xFFFFFu) | 0x100000u, 7) * sg;
-  const int      ml = (int)(lo & 0x1FFFFFFu) * (sg * 16);
-  FxAcc          p;
-  p.set(X.h, X.l, mh, ml, 0);
-  return fx_split(((p.hi << 2) + (p.mid >> 27)) >> s);
+  const unsigned ec = abs_hi(c) >> 20, ev = abs_hi(v) >> 20;
+  const int      t = (int)(ec + ev) - 1022;
+  return ec == 0u ? 0u : ev == 0x7FFu ? 0x7FFu : ev == 0u || t < 0 ? 0u : (unsigned)t;
 }
 
-// X C 2^-57 shifted down by `shift`, C = (ch, cl) of the same form
-__device__ __forceinline__ Limbs fx_times(Limbs X, Limbs C, int shift)
+// (-)c v 2^(57 - E) as limbs for top = E + 1022 >= fx_product_top(c, v)
+__device__ __forceinline__ Limbs fx_product(double c, double v, int top, bool negative)
 {
-  FxAcc p;
-  p.set(X.h, X.l, C.h, C.l, 0);
-  return fx_split(((p.hi << 2) + (p.mid >> 27)) >> shift);
+  const unsigned hc = (unsigned)__double2hiint(c), hv = (unsigned)__double2hiint(v);
+  const unsigned lc = (unsigned)__double2loint(c), lv = (unsigned)__double2loint(v);
+  const int      ec = (int)((hc << 1) >> 21), ev = (int)((hv << 1) >> 21);
+  // a factor of zero (or subnormal): shift everything out
+  const int      s = ec == 0 || ev == 0 ? 63 : min(top - (ec + ev - 1022), 63);
+  // mantissas of 58 and 57 bits as limbs of 29 and 28 + 29
+  const int      xh = (int)__funnelshift_l(lc, (hc & 0xFFFFFu) | 0x100000u, 8), xl = (int)((lc & 0xFFFFFFu) << 5);
+  const int      yh = (int)__funnelshift_l(lv, (hv & 0xFFFFFu) | 0x100000u, 7), yl = (int)((lv & 0x1FFFFFFu) << 4);
+  const long long mid = mad_wide(xl, yh, mad_wide(xh, yl, (long long)__umulhi((unsigned)xl << 3, (unsigned)yl)));
+  const int       sg  = ((int)(hc ^ hv) >> 31) | 1;
+  Limbs           r   = fx_split(((mul_wide(xh, yh) << 1) + (mid >> 28)) >> s);
+  r.h *= negative ? -sg : sg;
+  r.l *= negative ? -sg : sg;
+  return r;
+}
+
+// X W 2^-58 as limbs, |X| <= 2^57, |W| <= 2^58 (W: a metric value of the
+// cell geometry or a uniform constant, y 2^(58 - Ey) as limbs)
+__device__ __forceinline__ Limbs fx_times(Limbs X, int2 W)
+{
+  // the shift of mid rounds to nearest, and 2^28 is added to balance l
+  const long long hi  = mul_wide(X.h, W.x);
+  const long long mid = mad_wide(X.l, W.x, mad_wide(X.h, W.y, (1ll << 57) + (1ll << 28)));
+  const long long Y   = hi + (mid >> 29);
+  Limbs           r;
+  r.h = (int)(Y >> 29);
+  r.l = (int)((unsigned)Y & 0x1FFFFFFFu) - (1 << 28);
+  return r;
 }
 
 __device__ __forceinline__ unsigned long long fx_abs(long long x)
@@ -143,7 +172,7 @@ __device__ __forceinline__ double fx_to_double(long long Z, int e)
 // 2^62: 3 (||Dw||_inf + max_q (|lw0| + |lw1|)) 2^(57 + kFxGuard - kd) is at
 // most 2^61.4 for n = 2..7 (20.8, 39.7, 64.0, 93.9, 129.4, 170.6 for the
 // bracket).
-constexpr int kFxGuard = 2;
+constexpr int kFxGuard = 2, kFxShift = 1 + kFxGuard;
 template <int N>
 constexpr int fx_kd()
 {
@@ -152,23 +181,24 @@ constexpr int fx_kd()
 
 struct FxEvenOdd
 {
-  int2 e[3][3], o[3][3], ce[3], mid[3], cc;
+  FxConst e[3][3], o[3][3], ce[3], mid[3], cc;
 };
 
 struct FxTables
 {
   FxEvenOdd Dw;
-  int2      lwe[4], lwo[4];
+  FxConst   lwe[4], lwo[4];
 };
 
 static __constant__ FxTables c_tab_fx[kMaxNDev + 1];
 
 // c 2^bits as balanced limbs
-inline int2 fx_host_limbs(double c, int bits)
+inline FxConst fx_host_limbs(double c, int bits, int shift)
 {
   const long long X = llrint(ldexp(c, bits));
   const long long l = ((X + (1ll << 28)) & ((1ll << 29) - 1)) - (1ll << 28);
-  return make_int2((int)((X - l) >> 29), (int)l);
+  const long long h = (X - l) >> 29;
+  return FxConst{(int)h, (int)l, (int)(h << shift)};
 }
 
 inline cudaError_t upload_fx_local(const DevTables<double> *d)
@@ -184,26 +214,17 @@ inline cudaError_t upload_fx_local(const DevTables<double> *d)
         {
           for (int i = 0; i < h; ++i)
             {
-              t[n].Dw.e[q][i] = fx_host_limbs(M.e[q][i], bits);
-              t[n].Dw.o[q][i] = fx_host_limbs(M.o[q][i], bits);
+              t[n].Dw.e[q][i] = fx_host_limbs(M.e[q][i], bits, kFxShift);
+              t[n].Dw.o[q][i] = fx_host_limbs(M.o[q][i], bits, kFxShift);
             }
-          t[n].Dw.ce[q]  = fx_host_limbs(M.ce[q], bits);
-          t[n].Dw.mid[q] = fx_host_limbs(M.mid[q], bits);
-          t[n].lwo[q]    = fx_host_limbs(d[n].lwo[q], bits);
+          t[n].Dw.ce[q]  = fx_host_limbs(M.ce[q], bits, kFxShift);
+          t[n].Dw.mid[q] = fx_host_limbs(M.mid[q], bits, kFxShift);
+          t[n].lwo[q]    = fx_host_limbs(d[n].lwo[q], bits, kFxShift);
         }
       for (int q = 0; q < (n + 1) / 2; ++q)
-        t[n].lwe[q] = fx_host_limbs(d[n].lwe[q], bits);
+        t[n].lwe[q] = fx_host_limbs(d[n].lwe[q], bits, kFxShift);
     }
   return cudaMemcpyToSymbol(c_tab_fx, t, sizeof(t));
-}
-
-// Fixed-point value of an accumulator of products with table constants,
-// rounded to nearest (started with kFxHalf): a truncation's bias would be the
-// same in every stage and add up over the steps
-constexpr long long kFxHalf = 1ll << (27 - kFxGuard);
-__device__ __forceinline__ long long fx_value(const FxAcc &a)
-{
-  return (a.hi << (1 + kFxGuard)) + (a.mid >> (28 - kFxGuard));
 }
 
 // Volume and lift terms of one pencil: out = Dw V + lw0 F_lo + lw1 F_hi from
@@ -225,29 +246,29 @@ __device__ __forceinline__ void fx_sweep_lift(const FxTables &tb, const Limbs (&
 #pragma unroll
   for (int q = 0; q < H; ++q)
     {
-      FxAcc E, O;
-      O.set(psh, psl, tb.lwe[q].x, tb.lwe[q].y, kFxHalf);
-      E.set(pdh, pdl, tb.lwo[q].x, tb.lwo[q].y, kFxHalf);
+      FxAcc<kFxShift> E, O;
+      O.set(psh, psl, tb.lwe[q]);
+      E.set(pdh, pdl, tb.lwo[q]);
 #pragma unroll
       for (int i = 0; i < H; ++i)
         {
-          E.add(eh[i], el[i], tb.Dw.e[q][i].x, tb.Dw.e[q][i].y);
-          O.add(oh[i], ol[i], tb.Dw.o[q][i].x, tb.Dw.o[q][i].y);
+          E.add(eh[i], el[i], tb.Dw.e[q][i]);
+          O.add(oh[i], ol[i], tb.Dw.o[q][i]);
         }
       if (N % 2)
-        E.add(V[H].h, V[H].l, tb.Dw.ce[q].x, tb.Dw.ce[q].y);
-      const long long a = fx_value(O), b = fx_value(E);
+        E.add(V[H].h, V[H].l, tb.Dw.ce[q]);
+      const long long a = O.value(), b = E.value();
       out[q]         = a + b;
       out[N - 1 - q] = a - b;
     }
   if (N % 2)
     {
-      FxAcc m;
-      m.set(psh, psl, tb.lwe[H].x, tb.lwe[H].y, kFxHalf);
+      FxAcc<kFxShift> m;
+      m.set(psh, psl, tb.lwe[H]);
 #pragma unroll
       for (int i = 0; i < H; ++i)
-        m.add(oh[i], ol[i], tb.Dw.mid[i].x, tb.Dw.mid[i].y);
-      out[H] = fx_value(m);
+        m.add(oh[i], ol[i], tb.Dw.mid[i]);
+      out[H] = m.value();
     }
 }
 

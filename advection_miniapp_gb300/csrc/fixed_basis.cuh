@@ -11,7 +11,7 @@ namespace adv
 struct FxBasisTables
 {
   FxEvenOdd S, Si, St;
-  int2      l0[7], l1[7];
+  FxConst   l0[7], l1[7];
 };
 
 static __constant__ FxBasisTables c_tab_fxb[kMaxNDev + 1];
@@ -31,18 +31,18 @@ inline cudaError_t upload_fx_basis_local(const DevTables<double> *d)
             {
               for (int i = 0; i < h; ++i)
                 {
-                  to[m]->e[q][i] = fx_host_limbs(from[m]->e[q][i], 57);
-                  to[m]->o[q][i] = fx_host_limbs(from[m]->o[q][i], 57);
+                  to[m]->e[q][i] = fx_host_limbs(from[m]->e[q][i], 57, 2);
+                  to[m]->o[q][i] = fx_host_limbs(from[m]->o[q][i], 57, 2);
                 }
-              to[m]->ce[q]  = fx_host_limbs(from[m]->ce[q], 57);
-              to[m]->mid[q] = fx_host_limbs(from[m]->mid[q], 57);
+              to[m]->ce[q]  = fx_host_limbs(from[m]->ce[q], 57, 2);
+              to[m]->mid[q] = fx_host_limbs(from[m]->mid[q], 57, 2);
             }
-          to[m]->cc = fx_host_limbs(from[m]->cc, 57);
+          to[m]->cc = fx_host_limbs(from[m]->cc, 57, 2);
         }
       for (int q = 0; q < n; ++q)
         {
-          t[n].l0[q] = fx_host_limbs(d[n].l0[q], 56);
-          t[n].l1[q] = fx_host_limbs(d[n].l1[q], 56);
+          t[n].l0[q] = fx_host_limbs(d[n].l0[q], 56, 2);
+          t[n].l1[q] = fx_host_limbs(d[n].l1[q], 56, 2);
         }
     }
   return cudaMemcpyToSymbol(c_tab_fxb, t, sizeof(t));
@@ -54,10 +54,8 @@ inline cudaError_t upload_fx_basis_local(const DevTables<double> *d)
 template <int N>
 __device__ __forceinline__ void fx_sweep_sym(const FxEvenOdd &M, const Limbs (&X)[N], long long (&out)[N])
 {
-  constexpr int       H    = N / 2;
-  constexpr long long half = 1ll << 26;
-  auto                value = [](const FxAcc &a) { return (a.hi << 2) + (a.mid >> 27); };
-  int                 eh[H], el[H], oh[H], ol[H];
+  constexpr int H = N / 2;
+  int           eh[H], el[H], oh[H], ol[H];
 #pragma unroll
   for (int i = 0; i < H; ++i)
     {
@@ -67,29 +65,29 @@ __device__ __forceinline__ void fx_sweep_sym(const FxEvenOdd &M, const Limbs (&X
 #pragma unroll
   for (int q = 0; q < H; ++q)
     {
-      FxAcc E, O;
-      E.set(eh[0], el[0], M.e[q][0].x, M.e[q][0].y, half);
-      O.set(oh[0], ol[0], M.o[q][0].x, M.o[q][0].y, half);
+      FxAcc<2> E, O;
+      E.set(eh[0], el[0], M.e[q][0]);
+      O.set(oh[0], ol[0], M.o[q][0]);
 #pragma unroll
       for (int i = 1; i < H; ++i)
         {
-          E.add(eh[i], el[i], M.e[q][i].x, M.e[q][i].y);
-          O.add(oh[i], ol[i], M.o[q][i].x, M.o[q][i].y);
+          E.add(eh[i], el[i], M.e[q][i]);
+          O.add(oh[i], ol[i], M.o[q][i]);
         }
       if (N % 2)
-        E.add(X[H].h, X[H].l, M.ce[q].x, M.ce[q].y);
-      const long long a = value(E), b = value(O);
+        E.add(X[H].h, X[H].l, M.ce[q]);
+      const long long a = E.value(), b = O.value();
       out[q]         = a + b;
       out[N - 1 - q] = a - b;
     }
   if (N % 2)
     {
-      FxAcc m;
-      m.set(X[H].h, X[H].l, M.cc.x, M.cc.y, half);
+      FxAcc<2> m;
+      m.set(X[H].h, X[H].l, M.cc);
 #pragma unroll
       for (int i = 0; i < H; ++i)
-        m.add(eh[i], el[i], M.mid[i].x, M.mid[i].y);
-      out[H] = value(m);
+        m.add(eh[i], el[i], M.mid[i]);
+      out[H] = m.value();
     }
 }
 

@@ -28,7 +28,10 @@ struct adv_handle
   double  *d_cell_geo64    = nullptr;   // FP32 increments: the FP64 copy for the anchor stage
   double  *d_face_geo64[3] = {};
   int     *d_cell_exp    = nullptr;     // field geometry: exponent of the largest |vt| per cell
-  bool     fx_ok         = false;       // the metric is inside the block fixed-point window
+  // FP64 advection without a skew term on a metric inside the block
+  // fixed-point window: the stages run in that arithmetic, and vt in the FP64
+  // cell geometry is stored as limbs (fx_const58)
+  bool     fx_ok         = false;
   double  *d_face_x[3]   = {};
   double  *d_partials    = nullptr;
   double  *d_scratch[2]  = {};

@@ -61,6 +61,7 @@ struct StageArgs
   // or the uniform constants within 2^+-200), and in the field case the
   // largest biased binary64 exponent of vt per cell
   int           fx_ok;
+  int           vt_limbs; // field case: vt of cell_geo as limbs (fx_const58 with the cell's exponent)
   const int    *cell_exp;
   const void   *cell_geo;    // field case: [vt0|vt1|vt2|idet] x n^3 per cell (T)
   const void   *face_geo[3]; // field case: n^2 (P, M) pairs per face (T)

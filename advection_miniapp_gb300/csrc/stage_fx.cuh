@@ -55,6 +55,35 @@ __device__ __noinline__ void stage_gauss_masked(const StageArgs &A, long long ce
   stage_gauss_cta<N, double, UNI, false, TR, INC, UPW>(A, cell0, smem, mask);
 }
 
+// The traces of a pencil x that the next stage reads: at the low face if bit 0
+// of `own` is set, at the high face if bit 1 is.  A loop, so that one chain
+// serves lanes with either face and a second one runs only in warps that
+// have a pencil with both (as predicated code both would issue on the FP64 pipe).
+template <int N>
+__device__ __forceinline__ void write_traces(const DevTables<double> &tb, const double (&x)[N], unsigned own, double *to)
+{
+#pragma unroll 1
+  for (int s = own & 1u ? 0 : 1; s < (own & 2u ? 2 : 1); ++s)
+    {
+      const double *l = s ? tb.l1 : tb.l0;
+      double        h = l[0] * x[0];
+#pragma unroll
+      for (int q = 1; q < N; ++q)
+        h = fma(l[q], x[q], h);
+      to[s * N * N] = h;
+    }
+}
+
+// Dirichlet data at face point r of a face normal to d (out of line: rare, and
+// long with the exact solution)
+static __device__ __noinline__ double boundary_value(const StageArgs &A, int d, unsigned face, int r, int nf)
+{
+  if (!A.bc_exact)
+    return 0.0;
+  const double *x = (d == 0 ? A.face_x[0] : d == 1 ? A.face_x[1] : A.face_x[2]) + ((size_t)face * nf + r) * 3;
+  return exact_value(A.ex, x[0], x[1], x[2], A.t);
+}
+
 template <int N, bool UNI, bool TR, bool INC, bool UPW>
 __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long cell0, unsigned char *smem_raw)
 {
@@ -64,7 +93,7 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
   constexpr int NF = N * N;
   constexpr int NT = FS::THREADS;
   static_assert(!UPW || (TR && !UNI), "upwind traces are written on field geometry");
-  int2      *Ub    = reinterpret_cast<int2 *>(smem_raw);         // [C][NQ] U: binary64, then limbs
+  int2      *Ub    = reinterpret_cast<int2 *>(smem_raw);         // [C][NQ] U as limbs
   long long *Qb    = reinterpret_cast<long long *>(Ub + C * NQ); // [C][NQ] Z, then the next input
   double    *Gb    = reinterpret_cast<double *>(Qb + C * NQ);    // field: [C][4][NQ] geometry
   unsigned  *s_eu = reinterpret_cast<unsigned *>(Gb + (UNI ? 0 : 4 * C * NQ)), *s_ef = s_eu + C, *s_bad = s_ef + C;
@@ -125,105 +154,76 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
             }
         }
     }
-  if (!TR)
-    {
-      if (mine)
-        {
-#pragma unroll
-          for (int k = 0; k < N; ++k)
-            reinterpret_cast<double *>(Ub)[cl * NQ + r + k * NF] = U[k];
-        }
-    }
   __syncthreads();
 
-  // ---- face fluxes at the pencil's six face points, binary64
-  double   F[6];
-  unsigned own = 0; // upwind traces: bit j: the own trace of face j is read
+  // ---- face fluxes at the pencil's six face points as pairs of factors
+  //      c v: where one of P, M is zero (upwind flux) the other times the value
+  //      on its side, formed in fixed point below; else 1 times the binary64 flux.
+  //      Low face M u_own + P u_nbr, high face -(P u_own + M u_nbr).
+  double   fc[6], fv[6];
+  unsigned own = 0; // bit j: the own trace of face j is read
   if (mine)
     {
       unsigned mf = 0, mu = 0;
-      // Dirichlet data of face j
-      auto boundary = [&](int j) -> double {
-        if (!A.bc_exact)
-          return 0.0;
-        const double *x = A.face_x[j >> 1] + ((size_t)face[j] * NF + r) * 3;
-        return exact_value(A.ex, x[0], x[1], x[2], A.t);
+      // coefficients of the own and the neighbour's value at face j
+      auto co = [&](int j) { return (j & 1) ? P[j] : M[j]; };
+      auto cn = [&](int j) { return (j & 1) ? M[j] : P[j]; };
+      // value of cell c on its side of face j: its trace, or the contraction
+      // of its pencil in the order the traces are formed in
+      auto face_value = [&](long long c, bool self, int j) -> double {
+        if (TR)
+          return __ldg(tr_in + (c * 6 + (self ? j : j ^ 1)) * NF + r);
+        const int     st = j < 2 ? 1 : j < 4 ? N : NF;
+        const double *g  = A.r_in + c * NQ + (j < 2 ? N * r : j < 4 ? offy : r);
+        const double *l  = self == (bool)(j & 1) ? tb.l1 : tb.l0;
+        double        v[N], u;
+#pragma unroll
+        for (int q = 0; q < N; ++q)
+          v[q] = __ldg(g + q * st);
+        u = l[0] * v[0];
+#pragma unroll
+        for (int q = 1; q < N; ++q)
+          u = fma(l[q], v[q], u);
+        return u;
       };
-      if (UPW)
-        {
-          // one read per face point: the trace on the side whose coefficient
-          // is not zero (the own side: M of a low face, P of a high one)
-#pragma unroll
-          for (int j = 0; j < 6; ++j)
-            {
-              const bool      mine_j = nonzero((j & 1) ? P[j] : M[j]);
-              const long long c      = mine_j || nb[j] < 0 ? cell0 + cl : (long long)nb[j];
-              own |= mine_j ? 1u << j : 0u;
-              F[j] = __ldg(tr_in + (c * 6 + (mine_j || nb[j] < 0 ? j : j ^ 1)) * NF + r);
-            }
-#pragma unroll
-          for (int j = 0; j < 6; ++j)
-            {
-              if (nb[j] < 0 && !((own >> j) & 1))
-                F[j] = boundary(j);
-              F[j] = or_bits(P[j], M[j]) * F[j];
-            }
-        }
-      else
-        {
-          double uo[6], un[6];
-#pragma unroll
-          for (int j = 0; j < 6; ++j)
-            {
-              const int     d  = j >> 1;
-              const int     st = d == 0 ? 1 : d == 1 ? N : NF;
-              const int     at = d == 0 ? N * r : d == 1 ? offy : r;
-              if (TR)
-                {
-                  uo[j] = __ldg(tr_in + ((cell0 + cl) * 6 + j) * NF + r);
-                  un[j] = nb[j] < 0 ? boundary(j) : __ldg(tr_in + ((long long)nb[j] * 6 + (j ^ 1)) * NF + r);
-                }
-              else
-                {
-                  // contractions of the own pencil and of the neighbour's, in
-                  // the order the traces are formed in
-                  const double *p  = reinterpret_cast<const double *>(Ub) + cl * NQ + at;
-                  const double *lo = (j & 1) ? tb.l1 : tb.l0, *ln = (j & 1) ? tb.l0 : tb.l1;
-                  double        v[N];
-                  if (nb[j] >= 0)
-                    {
-#pragma unroll
-                      for (int q = 0; q < N; ++q)
-                        v[q] = __ldg(A.r_in + (long long)nb[j] * NQ + at + q * st);
-                    }
-                  uo[j] = lo[0] * p[0];
-#pragma unroll
-                  for (int q = 1; q < N; ++q)
-                    uo[j] = fma(lo[q], p[q * st], uo[j]);
-                  if (nb[j] < 0)
-                    un[j] = boundary(j);
-                  else
-                    {
-                      un[j] = ln[0] * v[0];
-#pragma unroll
-                      for (int q = 1; q < N; ++q)
-                        un[j] = fma(ln[q], v[q], un[j]);
-                    }
-                }
-            }
-          // as direction_pass_pm: low face M u_own + P u_nbr, high face
-          // -(P u_own + M u_nbr)
-#pragma unroll
-          for (int j = 0; j < 6; ++j)
-            F[j] = (j & 1) ? fma(P[j], uo[j], M[j] * un[j]) : fma(M[j], uo[j], P[j] * un[j]);
-        }
+      // one value per face point: the side whose coefficient is not zero
+      unsigned two = 0, edge = 0; // faces that need both, that take Dirichlet data
 #pragma unroll
       for (int j = 0; j < 6; ++j)
         {
-          if (j & 1)
-            F[j] = -F[j];
-          mf = max(mf, abs_hi(F[j]));
+          const bool ro = nonzero(co(j)), self = ro || nb[j] < 0;
+          own |= ro ? 1u << j : 0u;
+          edge |= !ro && nb[j] < 0 ? 1u << j : 0u;
+          if (!UPW)
+            two |= ro && nonzero(cn(j)) ? 1u << j : 0u;
+          fv[j] = face_value(self ? cell0 + cl : (long long)nb[j], self, j);
+          fc[j] = or_bits(P[j], M[j]);
         }
+      // a velocity that changes sign in time exchanges P and M between the
+      // stages: all traces are written for the next one
+      if (!UPW && !UNI)
+        own = 63u;
+      if (edge)
+        {
+#pragma unroll
+          for (int j = 0; j < 6; ++j)
+            if ((edge >> j) & 1u)
+              fv[j] = boundary_value(A, j >> 1, face[j], r, NF);
+        }
+      if (!UPW && two)
+        {
+#pragma unroll
+          for (int j = 0; j < 6; ++j)
+            if ((two >> j) & 1u)
+              {
+                const double un = nb[j] < 0 ? boundary_value(A, j >> 1, face[j], r, NF) : face_value(nb[j], false, j);
+                fv[j]           = fma(co(j), fv[j], cn(j) * un);
+                fc[j]           = 1.0;
+              }
+        }
+#pragma unroll
+      for (int j = 0; j < 6; ++j)
+        mf = max(mf, fx_product_top(fc[j], fv[j]));
 #pragma unroll
       for (int k = 0; k < N; ++k)
         mu = max(mu, abs_hi(U[k]));
@@ -233,24 +233,23 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
   __syncthreads();
 
   // ---- the block's scale: biased exponents of the tops of U, vt U and Z
-  Limbs f[6], cv[3];
+  Limbs f[6];
+  int2  cv[3];
   bool  live = mine;
-  int   topv = 0, topz = 0, dz = 0;
+  int   topz = 0;
   if (mine)
     {
       const unsigned mu = s_eu[cl], mf = s_ef[cl];
-      const int      eu = (int)(mu >> 20), ef = (int)(mf >> 20);
-      if (UNI)
-        topv = (int)(max(max(abs_hi(A.cv[0]), abs_hi(A.cv[1])), abs_hi(A.cv[2])) >> 20);
-      else
-        topv = A.cell_exp[cell0 + cl];
+      const int      eu = (int)(mu >> 20), ef = (int)mf;
+      const int topv = UNI ? (int)(max(max(abs_hi(A.cv[0]), abs_hi(A.cv[1])), abs_hi(A.cv[2])) >> 20)
+                           : A.cell_exp[cell0 + cl];
       const bool zero = (mu | mf) == 0;
       topz            = zero ? 1023 : max(eu + topv - 1022, ef);
       live            = eu < 1623 && ef < 1623 && topz > 623;
       if (!live && r == 0)
         atomicOr(s_bad, 1u << cl);
-      const int topu = max(eu, topz - topv + 1022 - 64);
-      dz             = topz - (topu + topv - 1022);
+      // U so that vt U is in Z's scale (topu >= eu)
+      const int topu = topz - topv + 1022;
       if (live)
         {
 #pragma unroll
@@ -261,12 +260,12 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
             }
 #pragma unroll
           for (int j = 0; j < 6; ++j)
-            f[j] = fx_from_double(F[j], topz);
+            f[j] = fx_product(fc[j], fv[j], topz, j & 1);
           if (UNI)
             {
 #pragma unroll
               for (int d = 0; d < 3; ++d)
-                cv[d] = fx_from_double(A.cv[d], topv);
+                cv[d] = fx_const58(A.cv[d], topv);
             }
         }
     }
@@ -275,7 +274,7 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
   __syncthreads();
 
   // one direction pass: the pencil at p (stride st) with vt at v (stride st)
-  auto pass = [&](const int2 *p, int st, const double *v, const Limbs &c, const Limbs &flo, const Limbs &fhi,
+  auto pass = [&](const int2 *p, int st, const double *v, const int2 &c, const Limbs &flo, const Limbs &fhi,
                   long long(&out)[N]) {
     Limbs V[N];
 #pragma unroll
@@ -284,7 +283,7 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
         const int2 u = p[k * st];
         Limbs      X;
         X.h = u.x, X.l = u.y;
-        V[k] = UNI ? fx_times(X, c, min(dz, 63)) : fx_times_double(X, v[k * st], topv + dz);
+        V[k] = fx_times(X, UNI ? c : reinterpret_cast<const int2 *>(v)[k * st]);
       }
     fx_sweep_lift<N>(fx, V, flo, fhi, out);
   };
@@ -323,71 +322,89 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
       pass(Ub + off, NF, G + 2 * NQ + r, cv[2], f[4], f[5], out);
       // Z = integer x 2^(topz - 1022 - 57 + kd - guard), times 1 / det J
       const int ez = topz - 1022 - 57 + fx_kd<N>() - kFxGuard;
-      double          next[N];
+      double    kd[N], next[N];
+      // (the mode's branches around whole loops: as predicated code the
+      // instructions of every mode would issue on the FP64 pipe)
 #pragma unroll
       for (int k = 0; k < N; ++k)
+        kd[k] = fx_to_double(Qb[off + k * NF] + out[k], ez);
+      if (!TR && !INC && A.mode == kModeVmult)
         {
-          const double    zi = fx_to_double(Qb[off + k * NF] + out[k], ez);
-          const long long gi = gb + k * NF;
-          if (!TR && !INC && A.mode == kModeVmult)
+          // implicit operator in weak form: JxW (c U - bracket), as stage_gauss_cta
+#pragma unroll
+          for (int k = 0; k < N; ++k)
             {
-              // implicit operator in weak form: JxW (c U - bracket), as stage_gauss_cta
               const double wq = tb.gw[r % N] * tb.gw[r / N] * tb.gw[k];
-              const double br = A.out_scale * zi, u = __ldg(A.r_in + gi);
-              A.r_out[gi]     = UNI ? wq * A.vol * (A.mass_factor * u - br)
-                                    : wq * (A.mass_factor * u / G[3 * NQ + r + k * NF] - br);
-              next[k]         = 0.0;
-              continue;
+              const double br = A.out_scale * kd[k], u = __ldg(A.r_in + gb + k * NF);
+              A.r_out[gb + k * NF] = UNI ? wq * A.vol * (A.mass_factor * u - br)
+                                         : wq * (A.mass_factor * u / G[3 * NQ + r + k * NF] - br);
             }
-          const double kd = UNI ? zi : zi * G[3 * NQ + r + k * NF];
+        }
+      else
+        {
+          if (!UNI)
+            {
+#pragma unroll
+              for (int k = 0; k < N; ++k)
+                kd[k] *= G[3 * NQ + r + k * NF];
+            }
           if (INC)
             {
               // the FP32 increments' FP64 anchor: K0 and the first G
-              A.k_out[gi]   = kd;
-              A.k_out32[gi] = d2f_int(kd);
-              A.r_out32[gi] = d2f_int(A.a * kd);
-              next[k]       = 0.0;
+#pragma unroll
+              for (int k = 0; k < N; ++k)
+                {
+                  A.k_out[gb + k * NF]   = kd[k];
+                  A.k_out32[gb + k * NF] = d2f_int(kd[k]);
+                  A.r_out32[gb + k * NF] = d2f_int(A.a * kd[k]);
+                }
             }
-          else if (A.mode == kModeStage)
+          else if (A.mode == kModeApply)
             {
-              const double kk = !TR && A.k_add ? kd + __ldcs(A.k_add + gi) : kd;
-              next[k]         = fma(A.a, kk, ui[k]);
-              A.u_out[gi]     = fma(A.b, kk, ui[k]);
-              A.r_out[gi]     = next[k];
-              if (!TR && A.k_out)
-                A.k_out[gi] = kk;
-            }
-          else if (A.mode == kModeLastStage)
-            {
-              const double kk = !TR && A.k_add ? kd + __ldcs(A.k_add + gi) : kd;
-              next[k]         = fma(A.b, kk, ui[k]);
-              if (!TR && A.u_base)
-                next[k] += A.u_base[gi];
-              A.u_out[gi] = next[k];
+#pragma unroll
+              for (int k = 0; k < N; ++k)
+                A.r_out[gb + k * NF] = A.out_scale * kd[k];
             }
           else
             {
-              A.r_out[gi] = A.out_scale * kd;
-              next[k]     = 0.0;
+              if (!TR && A.k_add)
+                {
+#pragma unroll
+                  for (int k = 0; k < N; ++k)
+                    kd[k] += __ldcs(A.k_add + gb + k * NF);
+                }
+#pragma unroll
+              for (int k = 0; k < N; ++k)
+                next[k] = fma(A.b, kd[k], ui[k]);
+              if (!TR && A.mode == kModeLastStage && A.u_base)
+                {
+#pragma unroll
+                  for (int k = 0; k < N; ++k)
+                    next[k] += A.u_base[gb + k * NF];
+                }
+#pragma unroll
+              for (int k = 0; k < N; ++k)
+                A.u_out[gb + k * NF] = next[k];
+              if (A.mode == kModeStage)
+                {
+#pragma unroll
+                  for (int k = 0; k < N; ++k)
+                    next[k] = fma(A.a, kd[k], ui[k]);
+#pragma unroll
+                  for (int k = 0; k < N; ++k)
+                    A.r_out[gb + k * NF] = next[k];
+                  if (!TR && A.k_out)
+                    {
+#pragma unroll
+                      for (int k = 0; k < N; ++k)
+                        A.k_out[gb + k * NF] = kd[k];
+                    }
+                }
             }
         }
       if (TR && !INC && A.tr_out)
         {
-          double *to = static_cast<double *>(A.tr_out) + ((cell0 + cl) * 6 + 4) * NF + r, lo, hi;
-          if (UPW)
-            {
-              if (upwind_pencil_traces<N, double>(tb, next, (own >> 4) & 1, (own >> 5) & 1, to, to + NF))
-                {
-                  pencil_traces<N, double>(tb, next, lo, hi);
-                  to[NF] = hi;
-                }
-            }
-          else
-            {
-              pencil_traces<N, double>(tb, next, lo, hi);
-              to[0]  = lo;
-              to[NF] = hi;
-            }
+          write_traces<N>(tb, next, own >> 4, static_cast<double *>(A.tr_out) + ((cell0 + cl) * 6 + 4) * NF + r);
 #pragma unroll
           for (int k = 0; k < N; ++k)
             Qb[off + k * NF] = __double_as_longlong(next[k]);
@@ -403,25 +420,12 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
             {
               const long long *p  = Qb + cl * NQ + (d == 0 ? N * r : offy);
               const int        st = d == 0 ? 1 : N;
-              double           x[N], lo, hi;
+              double           x[N];
 #pragma unroll
               for (int k = 0; k < N; ++k)
                 x[k] = __longlong_as_double(p[k * st]);
-              double *to = static_cast<double *>(A.tr_out) + ((cell0 + cl) * 6 + 2 * d) * NF + r;
-              if (UPW)
-                {
-                  if (upwind_pencil_traces<N, double>(tb, x, (own >> (2 * d)) & 1, (own >> (2 * d + 1)) & 1, to, to + NF))
-                    {
-                      pencil_traces<N, double>(tb, x, lo, hi);
-                      to[NF] = hi;
-                    }
-                }
-              else
-                {
-                  pencil_traces<N, double>(tb, x, lo, hi);
-                  to[0]  = lo;
-                  to[NF] = hi;
-                }
+              write_traces<N>(tb, x, own >> (2 * d),
+                              static_cast<double *>(A.tr_out) + ((cell0 + cl) * 6 + 2 * d) * NF + r);
             }
         }
     }

@@ -260,18 +260,17 @@ __device__ __forceinline__ void stage_fx_nodal_cta(const StageArgs &A, const lon
       for (int d = 0; d < 3; ++d)
         {
           load(Ub + (d == 0 ? ox : d == 1 ? oy : oz), d == 0 ? 1 : d == 1 ? N : NF);
-          FxAcc lo, hi;
-          lo.set(X[0].h, X[0].l, fxb.l0[0].x, fxb.l0[0].y, 1ll << 26);
-          hi.set(X[0].h, X[0].l, fxb.l1[0].x, fxb.l1[0].y, 1ll << 26);
+          FxAcc<2> lo, hi;
+          lo.set(X[0].h, X[0].l, fxb.l0[0]);
+          hi.set(X[0].h, X[0].l, fxb.l1[0]);
 #pragma unroll
           for (int q = 1; q < N; ++q)
             {
-              lo.add(X[q].h, X[q].l, fxb.l0[q].x, fxb.l0[q].y);
-              hi.add(X[q].h, X[q].l, fxb.l1[q].x, fxb.l1[q].y);
+              lo.add(X[q].h, X[q].l, fxb.l0[q]);
+              hi.add(X[q].h, X[q].l, fxb.l1[q]);
             }
-          // l is tabulated as c 2^56: the sums are at half a unit of X
-          const double uo[2] = {fx_to_double((lo.hi << 2) + (lo.mid >> 27), top3 - 1022 - 57),
-                                fx_to_double((hi.hi << 2) + (hi.mid >> 27), top3 - 1022 - 57)};
+          // l is tabulated as c 2^56: the sums are in units of X
+          const double uo[2] = {fx_to_double(lo.value(), top3 - 1022 - 57), fx_to_double(hi.value(), top3 - 1022 - 57)};
 #pragma unroll
           for (int s = 0; s < 2; ++s)
             {
@@ -303,7 +302,8 @@ __device__ __forceinline__ void stage_fx_nodal_cta(const StageArgs &A, const lon
 
   // ---- scale of vt U and the fluxes (as stage_fx_cta), direction passes
   int   topv = 0, topz = 0;
-  Limbs f[6], cv[3];
+  Limbs f[6];
+  int2  cv[3];
   int   dz = 0;
   if (live)
     {
@@ -318,7 +318,7 @@ __device__ __forceinline__ void stage_fx_nodal_cta(const StageArgs &A, const lon
           if (r == 0)
             atomicOr(s_bad, 1u << cl);
         }
-      dz = max(topz - (top3 + topv - 1022), 0);
+      dz = min(max(topz - (top3 + topv - 1022), 0), 63);
 #pragma unroll
       for (int j = 0; j < 6; ++j)
         f[j] = fx_from_double(F[j], topz);
@@ -326,16 +326,22 @@ __device__ __forceinline__ void stage_fx_nodal_cta(const StageArgs &A, const lon
         {
 #pragma unroll
           for (int d = 0; d < 3; ++d)
-            cv[d] = fx_from_double(A.cv[d], topv);
+            cv[d] = fx_const58(A.cv[d], topv);
         }
     }
   const double *G    = Gb + cl * 4 * NQ;
-  auto          pass = [&](const int2 *p, int st, const double *v, const Limbs &c, const Limbs &flo, const Limbs &fhi) {
+  auto          pass = [&](const int2 *p, int st, const double *v, const int2 &c, const Limbs &flo, const Limbs &fhi) {
     load(p, st);
     Limbs V[N];
 #pragma unroll
     for (int k = 0; k < N; ++k)
-      V[k] = UNI ? fx_times(X[k], c, min(dz, 63)) : fx_times_double(X[k], v[k * st], topv + dz);
+      V[k] = fx_times(X[k], UNI ? c : reinterpret_cast<const int2 *>(v)[k * st]);
+    if (dz) // the fluxes set the scale: cells of zeros or beside much larger ones
+      {
+#pragma unroll
+        for (int k = 0; k < N; ++k)
+          V[k] = fx_split((2 * ((long long)V[k].h * (1 << 29) + V[k].l)) >> dz);
+      }
     fx_sweep_lift<N>(fx, V, flo, fhi, T);
   };
   if (live)
@@ -432,30 +438,51 @@ __device__ __forceinline__ void stage_fx_nodal_cta(const StageArgs &A, const lon
       const int er = topr - 1022 - 58 + fx_si1<N>() + fx_si2<N>();
 #pragma unroll
       for (int k = 0; k < N; ++k)
+        x[k] = fx_to_double(T[k], er);
+      // (branches around whole loops, not predicated FP64 instructions)
+      if (!upd)
         {
-          const long long gi = gb + k * NF;
-          double          kd = fx_to_double(T[k], er);
-          if (weak)
-            A.r_out[gi] = kd;
-          else if (A.mode == kModeApply)
-            A.r_out[gi] = A.out_scale * kd;
-          else
+          if (!weak)
             {
-              if (A.k_add)
-                kd += __ldcs(A.k_add + gi);
-              double un = fma(A.b, kd, ui[k]);
-              if (A.mode == kModeLastStage)
+#pragma unroll
+              for (int k = 0; k < N; ++k)
+                x[k] *= A.out_scale;
+            }
+#pragma unroll
+          for (int k = 0; k < N; ++k)
+            A.r_out[gb + k * NF] = x[k];
+        }
+      else
+        {
+          if (A.k_add)
+            {
+#pragma unroll
+              for (int k = 0; k < N; ++k)
+                x[k] += __ldcs(A.k_add + gb + k * NF);
+            }
+          double un[N];
+#pragma unroll
+          for (int k = 0; k < N; ++k)
+            un[k] = fma(A.b, x[k], ui[k]);
+          if (A.mode == kModeLastStage && A.u_base)
+            {
+#pragma unroll
+              for (int k = 0; k < N; ++k)
+                un[k] += A.u_base[gb + k * NF];
+            }
+#pragma unroll
+          for (int k = 0; k < N; ++k)
+            A.u_out[gb + k * NF] = un[k];
+          if (A.mode == kModeStage)
+            {
+#pragma unroll
+              for (int k = 0; k < N; ++k)
+                A.r_out[gb + k * NF] = fma(A.a, x[k], ui[k]);
+              if (A.k_out)
                 {
-                  if (A.u_base)
-                    un += A.u_base[gi];
-                  A.u_out[gi] = un;
-                }
-              else
-                {
-                  A.u_out[gi] = un;
-                  A.r_out[gi] = fma(A.a, kd, ui[k]);
-                  if (A.k_out)
-                    A.k_out[gi] = kd;
+#pragma unroll
+                  for (int k = 0; k < N; ++k)
+                    A.k_out[gb + k * NF] = x[k];
                 }
             }
         }

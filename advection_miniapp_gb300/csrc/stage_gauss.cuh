@@ -202,6 +202,16 @@ __device__ __forceinline__ void stage_gauss_cta(const StageArgs &A, const long l
     return Fb + (cl * 6 + j) * 2 * NF;
   };
 
+  // uniform constants: whether the flux at face j has a zero coefficient on
+  // the own or the neighbour's trace (the block fixed-point stages do not
+  // write the traces that no flux reads)
+  auto trace_unread = [&](int j, bool own) -> bool {
+    if (!UNI || A.has_skew)
+      return false;
+    const T c = own == (bool)(j & 1) ? Consts<T>::P(A, j >> 1) : Consts<T>::M(A, j >> 1);
+    return !nonzero(c);
+  };
+
   // ---- phase 1: own values (one contiguous range of the CTA's cells) and
   //      the neighbours' values at the face points
   {
@@ -235,7 +245,7 @@ __device__ __forceinline__ void stage_gauss_cta(const StageArgs &A, const long l
       {
         const T *tr = static_cast<const T *>(A.tr_in) + cell0 * 6 * TRW * NF;
         for (int i = tid; i < ncell * 6 * TRW * NF; i += NT)
-          Tb[i] = __ldg(tr + i);
+          Tb[i] = trace_unread(i / (TRW * NF) % 6, true) ? T(0) : __ldg(tr + i);
       }
   }
   // the neighbours' values at the face points: one thread per face point
@@ -250,7 +260,7 @@ __device__ __forceinline__ void stage_gauss_cta(const StageArgs &A, const long l
           {
             // the neighbour's own trace on the shared face (its face j ^ 1)
             const T *tn      = static_cast<const T *>(A.tr_in) + ((long long)nb * 6 + (j ^ 1)) * TRW * NF + fq;
-            Nb[cf * NF + fq] = __ldg(tn);
+            Nb[cf * NF + fq] = trace_unread(j, false) ? T(0) : __ldg(tn);
             if (VISC)
               Nd[cf * NF + fq] = __ldg(tn + NF);
             return;
@@ -410,7 +420,8 @@ __device__ __forceinline__ void stage_gauss_cta(const StageArgs &A, const long l
           s_need[(cl * 6 + 0) * NF + r] = own_lo;
           s_need[(cl * 6 + 1) * NF + r] = own_hi;
           direction_pass_pm<N, T, UNI, VISC, 0, true, true>(A, tb, U, vlo, vhi, T(0), T(0), false, false, pm,
-                                                            geo(cl) + N * r, 1, out);
+                                                            geo(cl) + N * r, 1, out, T(0), T(0), T(0), T(0),
+                                                            vt_top(A, cell0 + cl));
         }
       else
         direction_pass<N, T, UNI, VISC, 0, TR>(A, tb, U, nbv(cl, 0, r), nbv(cl, 1, r), nbd(cl, 0, r),
@@ -418,7 +429,7 @@ __device__ __forceinline__ void stage_gauss_cta(const StageArgs &A, const long l
                                                faces(cl, 0), faces(cl, 1), geo(cl) + N * r, 1, out,
                                                TR ? trv(Tr, 0) : T(0), TR ? trv(Tr, TRW * NF) : T(0),
                                                TR && VISC ? trv(Tr, NF) : T(0),
-                                               TR && VISC ? trv(Tr, TRW * NF + NF) : T(0));
+                                               TR && VISC ? trv(Tr, TRW * NF + NF) : T(0), vt_top(A, cell0 + cl));
       T *z = Qb + cl * NQ + N * r;
 #pragma unroll
       for (int k = 0; k < N; ++k)
@@ -446,7 +457,8 @@ __device__ __forceinline__ void stage_gauss_cta(const StageArgs &A, const long l
           s_need[(cl * 6 + 2) * NF + r] = own_lo;
           s_need[(cl * 6 + 3) * NF + r] = own_hi;
           direction_pass_pm<N, T, UNI, VISC, 1, true, true>(A, tb, U, vlo, vhi, T(0), T(0), false, false, pm,
-                                                            geo(cl) + NQ + off, N, out);
+                                                            geo(cl) + NQ + off, N, out, T(0), T(0), T(0), T(0),
+                                                            vt_top(A, cell0 + cl));
         }
       else
         direction_pass<N, T, UNI, VISC, 1, TR>(A, tb, U, nbv(cl, 2, r), nbv(cl, 3, r), nbd(cl, 2, r),
@@ -454,7 +466,7 @@ __device__ __forceinline__ void stage_gauss_cta(const StageArgs &A, const long l
                                                faces(cl, 2), faces(cl, 3), geo(cl) + NQ + off, N, out,
                                                TR ? trv(Tr, 0) : T(0), TR ? trv(Tr, TRW * NF) : T(0),
                                                TR && VISC ? trv(Tr, NF) : T(0),
-                                               TR && VISC ? trv(Tr, TRW * NF + NF) : T(0));
+                                               TR && VISC ? trv(Tr, TRW * NF + NF) : T(0), vt_top(A, cell0 + cl));
       T *z = Qb + cl * NQ + off;
 #pragma unroll
       for (int k = 0; k < N; ++k)
@@ -483,7 +495,8 @@ __device__ __forceinline__ void stage_gauss_cta(const StageArgs &A, const long l
           T         vlo, vhi;
           upwind_values(cl, 4, r, pm, vlo, vhi, zlo, zhi);
           direction_pass_pm<N, T, UNI, VISC, 2, true, true>(A, tb, U, vlo, vhi, T(0), T(0), false, false, pm,
-                                                            G + 2 * NQ + r, NF, out);
+                                                            G + 2 * NQ + r, NF, out, T(0), T(0), T(0), T(0),
+                                                            vt_top(A, cell0 + cl));
         }
       else
         direction_pass<N, T, UNI, VISC, 2, TR>(A, tb, U, nbv(cl, 4, r), nbv(cl, 5, r), nbd(cl, 4, r),
@@ -491,7 +504,7 @@ __device__ __forceinline__ void stage_gauss_cta(const StageArgs &A, const long l
                                                faces(cl, 4), faces(cl, 5), G + 2 * NQ + r, NF, out,
                                                TR ? trv(Tr, 0) : T(0), TR ? trv(Tr, TRW * NF) : T(0),
                                                TR && VISC ? trv(Tr, NF) : T(0),
-                                               TR && VISC ? trv(Tr, TRW * NF + NF) : T(0));
+                                               TR && VISC ? trv(Tr, TRW * NF + NF) : T(0), vt_top(A, cell0 + cl));
       T              *z  = Qb + cl * NQ + r;
       const long long gb = (cell0 + cl) * NQ + r;
       double          next[N]; // the next stage's input along the pencil (traces)

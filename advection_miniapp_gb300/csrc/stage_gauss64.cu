@@ -1,7 +1,7 @@
 // Instantiations of the collocation-form stage kernel with a binary64
 // operator, and the change of basis of the fused LSRK loop.
 #include "fixed_basis.cuh"
-#include "stage_gauss.cuh"
+#include "stage_fx.cuh"
 
 namespace adv
 {
@@ -189,11 +189,7 @@ __global__ void __launch_bounds__(StageShape<N, double, true, false>::THREADS)
           double *to = traces + ((cell0 + cl) * 6 + 2 * d) * width * NF + r;
           if (UPW)
             {
-              if (upwind_pencil_traces<N, double>(tb, v, (own >> (2 * d)) & 1, (own >> (2 * d + 1)) & 1, to, to + NF))
-                {
-                  pencil_traces<N, double>(tb, v, lo, hi);
-                  to[NF] = hi;
-                }
+              write_traces<N>(tb, v, own >> (2 * d), to);
               continue;
             }
           pencil_traces<N, double>(tb, v, lo, hi);

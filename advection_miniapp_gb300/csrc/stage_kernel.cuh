@@ -315,15 +315,33 @@ __device__ __forceinline__ FacePM<T> face_pm(const StageArgs &A, const T *Flo, c
 // the nonzero coefficient of the low / high face (or zero) and nlo / nhi the
 // value on the upwind side there, own or neighbour; the flux is then one
 // product per face, with the same value as the general form.
+// exponent of a cell's vt limbs
+__device__ __forceinline__ int vt_top(const StageArgs &A, long long c)
+{
+  return A.vt_limbs ? A.cell_exp[c] : 0;
+}
+
 template <int N, typename T, bool UNI, bool VISC, int D, bool OWN_TR = false, bool UPW = false>
 __device__ __forceinline__ void direction_pass_pm(const StageArgs &A, const DevTables<T> &tb,
                                                   const T (&U)[N], T nlo, T nhi, T dnlo, T dnhi, bool blo,
                                                   bool bhi, const FacePM<T> &pm, const T *vt, int vstride,
                                                   T (&out)[N], T tr_lo = T(0), T tr_hi = T(0),
-                                                  T dtr_lo = T(0), T dtr_hi = T(0))
+                                                  T dtr_lo = T(0), T dtr_hi = T(0), int vtop = 0)
 {
   constexpr int NF = N * N;
   static_assert(!UPW || (OWN_TR && !VISC), "the upwind form takes its face values from the caller");
+  // vt at point q of the pencil (limbs: the cell geometry of the block
+  // fixed-point kernels, whose cells outside their window run here)
+  auto vtq = [&](int q) -> T {
+    if constexpr (sizeof(T) == sizeof(double) && !VISC)
+      if (A.vt_limbs)
+        {
+          const double w = vt[q * vstride];
+          return ((double)__double2loint(w) * 536870912.0 + (double)__double2hiint(w)) *
+                 __hiloint2double((vtop - 57) << 20, 0);
+        }
+    return vt[q * vstride];
+  };
   T ulo, uhi;
   if (OWN_TR)
     ulo = tr_lo, uhi = tr_hi;
@@ -378,11 +396,11 @@ __device__ __forceinline__ void direction_pass_pm(const StageArgs &A, const DevT
 #pragma unroll
           for (int i = 0; i < H; ++i)
             {
-              const T p = vt[(N - 1 - i) * vstride] * U[N - 1 - i];
-              e[i]      = fma(vt[i * vstride], U[i], p);
-              o[i]      = fma(vt[i * vstride], U[i], -p);
+              const T p = vtq(N - 1 - i) * U[N - 1 - i];
+              e[i]      = fma(vtq(i), U[i], p);
+              o[i]      = fma(vtq(i), U[i], -p);
             }
-          sweep_eo_anti_lift_parts<N, T>(tb.Dw_eo, e, o, N % 2 ? vt[H * vstride] * U[H] : T(0), phlo, phhi,
+          sweep_eo_anti_lift_parts<N, T>(tb.Dw_eo, e, o, N % 2 ? vtq(H) * U[H] : T(0), phlo, phhi,
                                          tb.lwe, tb.lwo, out);
           return;
         }
@@ -390,7 +408,7 @@ __device__ __forceinline__ void direction_pass_pm(const StageArgs &A, const DevT
 #pragma unroll
       for (int q = 0; q < N; ++q)
         {
-          const T c = UNI ? cvd : vt[q * vstride];
+          const T c = UNI ? cvd : vtq(q);
           w[q]      = A.has_skew ? (T(1) - sk) * (c * U[q]) : c * U[q];
         }
       sweep_eo_anti_lift<N, T>(tb.Dw_eo, w, phlo, phhi, tb.lwe, tb.lwo, out);
@@ -399,7 +417,7 @@ __device__ __forceinline__ void direction_pass_pm(const StageArgs &A, const DevT
           sweep2<N, T, true>(tb.D, tb.D_eo, U, du);
 #pragma unroll
           for (int q = 0; q < N; ++q)
-            out[q] = fma(-sk * (UNI ? cvd : vt[q * vstride]), du[q], out[q]);
+            out[q] = fma(-sk * (UNI ? cvd : vtq(q)), du[q], out[q]);
         }
       return;
     }
@@ -443,13 +461,13 @@ __device__ __forceinline__ void direction_pass_pm(const StageArgs &A, const DevT
       sweep2<N, T, true>(tb.D, tb.D_eo, U, du);
 #pragma unroll
       for (int q = 0; q < N; ++q)
-        w[q] = fma(adv, vt[q * vstride] * U[q], -cd * du[q]);
+        w[q] = fma(adv, vtq(q) * U[q], -cd * du[q]);
       sweep_eo_anti_lift<N, T, true>(tb.Dw_eo, w, phlo, phhi, tb.lwe, tb.lwo, out, dlo, dhi, tb.lde, tb.ldo);
       if (A.has_skew)
         {
 #pragma unroll
           for (int q = 0; q < N; ++q)
-            out[q] = fma(-sk * sa, vt[q * vstride] * du[q], out[q]);
+            out[q] = fma(-sk * sa, vtq(q) * du[q], out[q]);
         }
       return;
     }
@@ -462,7 +480,7 @@ __device__ __forceinline__ void direction_pass_pm(const StageArgs &A, const DevT
 #pragma unroll
   for (int q = 0; q < N; ++q)
     {
-      vtv[q] = UNI ? T(1) : vt[q * vstride];
+      vtv[q] = UNI ? T(1) : vtq(q);
       w[q]   = UNI ? U[q] : vtv[q] * U[q];
       if (VISC)
         w[q] = fma(adv, w[q], -Consts<T>::cdiff(A, D) * du[q]);
@@ -496,11 +514,11 @@ __device__ __forceinline__ void direction_pass(const StageArgs &A, const DevTabl
                                                const T (&U)[N], T nlo, T nhi, T dnlo, T dnhi, bool blo,
                                                bool bhi, int fq, const T *Flo, const T *Fhi, const T *vt,
                                                int vstride, T (&out)[N], T tr_lo = T(0), T tr_hi = T(0),
-                                               T dtr_lo = T(0), T dtr_hi = T(0))
+                                               T dtr_lo = T(0), T dtr_hi = T(0), int vtop = 0)
 {
   direction_pass_pm<N, T, UNI, VISC, D, OWN_TR>(A, tb, U, nlo, nhi, dnlo, dnhi, blo, bhi,
                                                 face_pm<T, UNI, D>(A, Flo, Fhi, fq), vt, vstride, out, tr_lo,
-                                                tr_hi, dtr_lo, dtr_hi);
+                                                tr_hi, dtr_lo, dtr_hi, vtop);
 }
 
 // Neighbour cells (-1 on boundary faces) and face ids of the cells
@@ -791,7 +809,7 @@ __device__ __forceinline__ void stage_cta(const StageArgs &A, const long long ce
                                          VISC ? Nd[(cl * 6 + 0) * NF + r] : T(0),
                                          VISC ? Nd[(cl * 6 + 1) * NF + r] : T(0),
                                          s_nbr[cl * 6 + 0] < 0, s_nbr[cl * 6 + 1] < 0, r,
-                                   F, Fh, Gb + cl * 4 * NQ + N * r, 1, out);
+                                   F, Fh, Gb + cl * 4 * NQ + N * r, 1, out, T(0), T(0), T(0), T(0), vt_top(A, cell0 + cl));
       T *z = Qb + cl * NQ + N * r;
 #pragma unroll
       for (int k = 0; k < N; ++k)
@@ -814,7 +832,8 @@ __device__ __forceinline__ void stage_cta(const StageArgs &A, const long long ce
                                          VISC ? Nd[(cl * 6 + 2) * NF + r] : T(0),
                                          VISC ? Nd[(cl * 6 + 3) * NF + r] : T(0),
                                          s_nbr[cl * 6 + 2] < 0, s_nbr[cl * 6 + 3] < 0, r,
-                                   F, Fh, Gb + (cl * 4 + 1) * NQ + off, N, out);
+                                   F, Fh, Gb + (cl * 4 + 1) * NQ + off, N, out, T(0), T(0), T(0), T(0),
+                                   vt_top(A, cell0 + cl));
       T *z = Qb + cl * NQ + off;
 #pragma unroll
       for (int k = 0; k < N; ++k)
@@ -837,7 +856,7 @@ __device__ __forceinline__ void stage_cta(const StageArgs &A, const long long ce
                                          VISC ? Nd[(cl * 6 + 4) * NF + r] : T(0),
                                          VISC ? Nd[(cl * 6 + 5) * NF + r] : T(0),
                                          s_nbr[cl * 6 + 4] < 0, s_nbr[cl * 6 + 5] < 0, r,
-                                   F, Fh, G + 2 * NQ + r, NF, out);
+                                   F, Fh, G + 2 * NQ + r, NF, out, T(0), T(0), T(0), T(0), vt_top(A, cell0 + cl));
       T *z = Qb + cl * NQ + r;
       if (A.mode != kModeVmult)
         {

@@ -166,3 +166,29 @@ def test_stage_in_place_outside_the_window(cuda, oracle_mod, adv_lib):
     op.perform_stage(0.0, 0.013, 0.021, r, k, u, r)
     assert np.abs(u.cpu().numpy() - uo).max() <= TOL * np.abs(uo).max()
     assert np.abs(r.cpu().numpy() - ro).max() <= TOL * np.abs(ro).max()
+
+
+@pytest.mark.parametrize("degree", [1, 4, 5])
+@pytest.mark.parametrize("curved", [0, 1])
+def test_step_across_the_sign_change_of_the_velocity(cuda, oracle_mod, adv_lib, curved, degree):
+    """cos(pi t / 0.5) changes sign at t = 0.25: the upwind side changes
+    between the stage that writes a trace and the one that reads it."""
+    cfg = dict(MESHES["rotating"], degree=degree, mesh_type=curved, deformation=0.05 * curved)
+    u0 = np.random.default_rng(degree).standard_normal(oracle_mod.Oracle(**cfg).n_dofs)
+    ref = oracle_step(oracle_mod, cfg, u0, 0.2495, 0.002)
+    got = gpu_step(cuda, adv_lib, cfg, u0, 0.2495, 0.002)
+    assert np.abs(got - ref).max() <= TOL * np.abs(ref).max()
+
+
+def test_uniform_velocity_with_a_zero_component(cuda, oracle_mod, adv_lib):
+    """No flux along y reads a trace; the binary64 path (first scale) must not
+    use the ones that were never written either."""
+    cfg = dict(MESHES["uniform"], degree=3, velocity=(0.7, 0.0, -0.4))
+    u0 = np.random.default_rng(12).standard_normal(oracle_mod.Oracle(**cfg).n_dofs)
+    ref = oracle_step(oracle_mod, cfg, u0, 0.0, 0.004)
+    for exponent in (-600, 0):
+        junk = cuda.full((1 << 22,), float("nan"), dtype=cuda.float64, device="cuda")  # memory the traces may get
+        del junk
+        cuda.cuda.empty_cache()
+        got = np.ldexp(gpu_step(cuda, adv_lib, cfg, np.ldexp(u0, exponent), 0.0, 0.004), -exponent)
+        assert np.abs(got - ref).max() <= TOL * np.abs(ref).max()
