@@ -168,6 +168,7 @@ int ensure_tables(int device)
   ADV_CUDA(adv::upload_tables_diag(td, tf));
   ADV_CUDA(adv::upload_tables_implicit(td, tf));
   ADV_CUDA(adv::upload_tables_batch(td, tf));
+  ADV_CUDA(adv::upload_tables_fx_visc(td, tf));
   ADV_CUDA(adv::upload_tables_fx_a(td, tf));
   ADV_CUDA(adv::upload_tables_fx_b(td, tf));
   ADV_CUDA(adv::upload_tables_fx_c(td, tf));
@@ -233,6 +234,18 @@ int upload_array(const std::vector<double> &src, void **dst, int64_t &bytes)
   ADV_CUDA(cudaMemcpy(*dst, tmp.data(), nb, cudaMemcpyHostToDevice));
   bytes += (int64_t)nb;
   return ADV_OK;
+}
+
+// SIPG constants (base_args) within the block fixed-point window
+bool sipg_in_fx_window(const adv_config &c, const adv::Mesh &m)
+{
+  bool ok = true;
+  for (int d = 0; d < 3; ++d)
+    {
+      const double k = c.diffusion * m.h[0] * m.h[1] * m.h[2] / (m.h[d] * m.h[d]);
+      ok             = ok && adv::in_fx_window(k) && adv::in_fx_window(k * c.penalty_factor);
+    }
+  return ok;
 }
 
 // vt of the field geometry in the form the block fixed-point kernels read
@@ -355,6 +368,7 @@ adv::StageArgs base_args(const adv_handle &h, double t, int prec = -1)
   A.fx_ok    = h.fx_ok;
   A.cell_exp = h.d_cell_exp;
   A.vt_limbs = h.fx_ok;
+  A.fx_visc  = h.fx_visc;
   A.t        = t;
   A.ex       = h.diag.ex;
   const double s = time_factor(h, t);
@@ -616,7 +630,9 @@ int create_handle(const adv_config *cfg, int z_begin, int z_end, adv_handle **ou
       const bool both = h->cfg.precision == ADV_PRECISION_FP32_INCREMENT;
       // the block fixed-point stages: every form with an FP64 operator
       h->fx_ok = g.fx_ok && (fp64 || both) && h->cfg.diffusion == 0.0 && h->cfg.factor_skew == 0.0;
-      if (h->fx_ok && !g.cell_exp.empty())
+      h->fx_visc = g.fx_ok && fp64 && h->cfg.diffusion != 0.0 && h->cfg.factor_skew == 0.0 &&
+                   sipg_in_fx_window(h->cfg, h->mesh);
+      if ((h->fx_ok || h->fx_visc) && !g.cell_exp.empty())
         {
           const size_t nb = g.cell_exp.size() * sizeof(int);
           if ((e = cudaMalloc(&h->d_cell_exp, nb)) != cudaSuccess ||
@@ -1239,10 +1255,12 @@ int run_steps(adv_handle *h, int n_steps, int ns, bool gauss, bool traces, doubl
   const int     n  = h->mesh.n;
   double       *tr_basis = traces ? static_cast<double *>(h->d_traces[0]) : nullptr;
   // the traces the first stage reads: only the upwind ones where it reads those
-  adv::StageArgs upw;
-  if (traces && upwind_traces(*h))
+  // (with diffusion: formed as the block fixed-point stages form them)
+  const bool           tr_args = traces && (upwind_traces(*h) || h->fx_visc);
+  adv::StageArgs       upw;
+  if (tr_args)
     upw = base_args(*h, 0.0, 0);
-  const adv::StageArgs *tr_upwind = traces && upwind_traces(*h) ? &upw : nullptr;
+  const adv::StageArgs *tr_upwind = tr_args ? &upw : nullptr;
   HostChunks    ch;
   int           nch = 0;
   if (host)

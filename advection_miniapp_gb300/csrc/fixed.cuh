@@ -201,7 +201,9 @@ inline FxConst fx_host_limbs(double c, int bits, int shift)
   return FxConst{(int)h, (int)l, (int)(h << shift)};
 }
 
-inline cudaError_t upload_fx_local(const DevTables<double> *d)
+// (static: every translation unit fills its own copy of the symbol.)
+// shift: that of the accumulators the translation unit's kernels use
+static inline cudaError_t upload_fx_local(const DevTables<double> *d, int shift = kFxShift)
 {
   static FxTables t[kMaxNDev + 1];
   memset(t, 0, sizeof(t));
@@ -214,15 +216,15 @@ inline cudaError_t upload_fx_local(const DevTables<double> *d)
         {
           for (int i = 0; i < h; ++i)
             {
-              t[n].Dw.e[q][i] = fx_host_limbs(M.e[q][i], bits, kFxShift);
-              t[n].Dw.o[q][i] = fx_host_limbs(M.o[q][i], bits, kFxShift);
+              t[n].Dw.e[q][i] = fx_host_limbs(M.e[q][i], bits, shift);
+              t[n].Dw.o[q][i] = fx_host_limbs(M.o[q][i], bits, shift);
             }
-          t[n].Dw.ce[q]  = fx_host_limbs(M.ce[q], bits, kFxShift);
-          t[n].Dw.mid[q] = fx_host_limbs(M.mid[q], bits, kFxShift);
-          t[n].lwo[q]    = fx_host_limbs(d[n].lwo[q], bits, kFxShift);
+          t[n].Dw.ce[q]  = fx_host_limbs(M.ce[q], bits, shift);
+          t[n].Dw.mid[q] = fx_host_limbs(M.mid[q], bits, shift);
+          t[n].lwo[q]    = fx_host_limbs(d[n].lwo[q], bits, shift);
         }
       for (int q = 0; q < (n + 1) / 2; ++q)
-        t[n].lwe[q] = fx_host_limbs(d[n].lwe[q], bits, kFxShift);
+        t[n].lwe[q] = fx_host_limbs(d[n].lwe[q], bits, shift);
     }
   return cudaMemcpyToSymbol(c_tab_fx, t, sizeof(t));
 }

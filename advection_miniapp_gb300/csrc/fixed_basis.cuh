@@ -16,7 +16,7 @@ struct FxBasisTables
 
 static __constant__ FxBasisTables c_tab_fxb[kMaxNDev + 1];
 
-inline cudaError_t upload_fx_basis_local(const DevTables<double> *d)
+static inline cudaError_t upload_fx_basis_local(const DevTables<double> *d)
 {
   static FxBasisTables t[kMaxNDev + 1];
   memset(t, 0, sizeof(t));

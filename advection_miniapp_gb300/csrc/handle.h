@@ -32,6 +32,7 @@ struct adv_handle
   // fixed-point window: the stages run in that arithmetic, and vt in the FP64
   // cell geometry is stored as limbs (fx_const58)
   bool     fx_ok         = false;
+  bool     fx_visc       = false; // FP64 collocation stages with diffusion run in it too (vt binary64)
   double  *d_face_x[3]   = {};
   double  *d_partials    = nullptr;
   double  *d_scratch[2]  = {};

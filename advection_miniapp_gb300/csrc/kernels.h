@@ -61,6 +61,7 @@ struct StageArgs
   // or the uniform constants within 2^+-200), and in the field case the
   // largest biased binary64 exponent of vt per cell
   int           fx_ok;
+  int           fx_visc;  // the same for the diffusive stages (vt stays binary64 there)
   int           vt_limbs; // field case: vt of cell_geo as limbs (fx_const58 with the cell's exponent)
   const int    *cell_exp;
   const void   *cell_geo;    // field case: [vt0|vt1|vt2|idet] x n^3 per cell (T)
@@ -116,6 +117,8 @@ cudaError_t launch_stage_fx_c(int n, const StageArgs &args, cudaStream_t stream)
 cudaError_t launch_stage_fx_nodal_a(int n, const StageArgs &args, cudaStream_t stream);
 cudaError_t launch_stage_fx_nodal_b(int n, const StageArgs &args, cudaStream_t stream);
 cudaError_t launch_stage_fx_nodal_c(int n, const StageArgs &args, cudaStream_t stream);
+cudaError_t launch_stage_fx_visc(int n, const StageArgs &args, cudaStream_t stream);
+cudaError_t upload_tables_fx_visc(const DevTables<double> *d, const DevTables<float> *f);
 cudaError_t upload_tables_fx_a(const DevTables<double> *d, const DevTables<float> *f);
 cudaError_t upload_tables_fx_b(const DevTables<double> *d, const DevTables<float> *f);
 cudaError_t upload_tables_fx_c(const DevTables<double> *d, const DevTables<float> *f);
@@ -127,7 +130,8 @@ cudaError_t upload_tables_gauss32(const DevTables<double> *d, const DevTables<fl
 // also writes the face traces of the result in the layout of StageArgs::tr_in
 // (width 2: values and reference normal derivatives, for SIPG).  upwind
 // (width 1): only the traces an upwind-trace stage reads (StageArgs::
-// upwind_tr), with the mesh and the FP64 face coefficients of *upwind.
+// upwind_tr), with the mesh and the FP64 face coefficients of *upwind; (width
+// 2) traces as the block fixed-point stages form them (upwind->fx_visc).
 cudaError_t launch_basis_change(int n, double *u, long long cell_begin, long long cell_end, bool to_gauss,
                                 cudaStream_t stream, double *traces = nullptr, int width = 1,
                                 const StageArgs *upwind = nullptr);

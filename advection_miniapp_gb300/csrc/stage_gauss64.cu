@@ -2,6 +2,7 @@
 // operator, and the change of basis of the fused LSRK loop.
 #include "fixed_basis.cuh"
 #include "stage_fx.cuh"
+#include "stage_fx_visc.cuh"
 
 namespace adv
 {
@@ -192,6 +193,18 @@ __global__ void __launch_bounds__(StageShape<N, double, true, false>::THREADS)
               write_traces<N>(tb, v, own >> (2 * d), to);
               continue;
             }
+          if (width == 2 && F.fx_visc)
+            {
+              // as the block fixed-point stages form them
+              ViscPencil<N> p2;
+              p2.set(v);
+              const double2 a = p2.at(tb, c_tab_fxv[N - 2], v, 0), b = p2.at(tb, c_tab_fxv[N - 2], v, 1);
+              to[0]      = a.x;
+              to[NF]     = a.y;
+              to[2 * NF] = b.x;
+              to[3 * NF] = b.y;
+              continue;
+            }
           pencil_traces<N, double>(tb, v, lo, hi);
           to[0]          = lo;
           to[width * NF] = hi;
@@ -238,7 +251,9 @@ cudaError_t launch_basis_n(double *u, long long cell_begin, long long cell_end, 
 cudaError_t upload_tables_gauss64(const DevTables<double> *d, const DevTables<float> *f)
 {
   cudaError_t e = upload_tables_local(d, f);
-  return e != cudaSuccess ? e : upload_fx_basis_local(d);
+  if (e == cudaSuccess)
+    e = upload_fx_basis_local(d);
+  return e != cudaSuccess ? e : upload_fx_visc_local(d);
 }
 
 cudaError_t launch_stage_gauss_fp64(int n, const StageArgs &args, cudaStream_t stream)
@@ -249,6 +264,8 @@ cudaError_t launch_stage_gauss_fp64(int n, const StageArgs &args, cudaStream_t s
     return n <= 3 ? launch_stage_fx_a(n, args, stream)
          : n <= 5 ? launch_stage_fx_b(n, args, stream)
                   : launch_stage_fx_c(n, args, stream);
+  if (args.fx_visc && !args.inc32 && args.mode != kModeVmult && !args.k_add && !args.k_out && !args.u_base)
+    return launch_stage_fx_visc(n, args, stream);
   return launch_stage_gauss_any<double>(n, args, stream);
 }
 

@@ -192,3 +192,50 @@ def test_uniform_velocity_with_a_zero_component(cuda, oracle_mod, adv_lib):
         cuda.cuda.empty_cache()
         got = np.ldexp(gpu_step(cuda, adv_lib, cfg, np.ldexp(u0, exponent), 0.0, 0.004), -exponent)
         assert np.abs(got - ref).max() <= TOL * np.abs(ref).max()
+
+
+# ---- advection-diffusion
+
+SIPG = {
+    "sipg-rotating": dict(n_cells=(3, 2, 3), periodic=0, velocity_type=1, velocity=(1.0, 1.0, 0.3), velocity_period=0.5,
+                          diffusion=1e-2, initial_condition=1, ic_params=(0.3, 0.5, 0.5, 0.2), boundary_value=0),
+    "sipg-periodic": dict(n_cells=(2, 3, 4), diffusion=3e-2),
+    "sipg-exact": dict(n_cells=(2, 2, 3), periodic=0, diffusion=1e-3, initial_condition=2, boundary_value=1),
+}
+
+
+@pytest.mark.parametrize("degree", [1, 2, 3, 4, 5, 6])
+@pytest.mark.parametrize("mesh", sorted(SIPG))
+def test_diffusive_step_matches_oracle(cuda, oracle_mod, adv_lib, mesh, degree):
+    cfg = dict(SIPG[mesh], degree=degree)
+    o = oracle_mod.Oracle(**cfg)
+    u0 = np.random.default_rng(degree).standard_normal(o.n_dofs)
+    dt = o.time_step(0.2)
+    # the sign change of the rotating velocity falls between the stages
+    ref = oracle_step(oracle_mod, cfg, u0, 0.2499, dt)
+    got = gpu_step(cuda, adv_lib, cfg, u0, 0.2499, dt)
+    assert np.abs(got - ref).max() <= TOL * np.abs(ref).max()
+    np.testing.assert_array_equal(
+        got, gpu_step(cuda, adv_lib, cfg, u0, 0.2499, dt, fused_form=adv_lib.FORM_COLLOCATION_NO_TRACES))
+
+
+@pytest.mark.parametrize("exponent", [-900, -300, 300, 900])
+def test_diffusive_step_commutes_with_powers_of_two(cuda, oracle_mod, adv_lib, exponent):
+    cfg = dict(SIPG["sipg-rotating"], degree=4)
+    o = oracle_mod.Oracle(**cfg)
+    u0 = np.random.default_rng(3).standard_normal(o.n_dofs)
+    dt = o.time_step(0.2)
+    ref = oracle_step(oracle_mod, cfg, u0, 0.0, dt)
+    got = np.ldexp(gpu_step(cuda, adv_lib, cfg, np.ldexp(u0, exponent), 0.0, dt), -exponent)
+    assert np.abs(got - ref).max() <= TOL * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("velocity, diffusion", [((0.0, 0.0, 0.0), 1e-2), ((1e-9, 0.0, 0.0), 1.0), ((1.0, 2.0, 0.0), 1e-12)])
+def test_diffusive_step_scales_of_the_terms(cuda, oracle_mod, adv_lib, velocity, diffusion):
+    """Pure diffusion, negligible advection, negligible diffusion."""
+    cfg = dict(degree=4, n_cells=(3, 3, 2), velocity=velocity, diffusion=diffusion)
+    u0 = np.random.default_rng(4).standard_normal(oracle_mod.Oracle(**cfg).n_dofs)
+    dt = 1e-5
+    ref = oracle_step(oracle_mod, cfg, u0, 0.0, dt)
+    got = gpu_step(cuda, adv_lib, cfg, u0, 0.0, dt)
+    assert np.abs(got - ref).max() <= TOL * np.abs(ref).max()
