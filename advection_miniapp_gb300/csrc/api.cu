@@ -1261,6 +1261,7 @@ int run_steps(adv_handle *h, int n_steps, int ns, bool gauss, bool traces, doubl
   if (tr_args)
     upw = base_args(*h, 0.0, 0);
   const adv::StageArgs *tr_upwind = tr_args ? &upw : nullptr;
+  const bool            fixed     = h->cfg.precision != ADV_PRECISION_FP32_OPERATOR;
   HostChunks    ch;
   int           nch = 0;
   if (host)
@@ -1315,7 +1316,7 @@ int run_steps(adv_handle *h, int n_steps, int ns, bool gauss, bool traces, doubl
           if (gauss)
             {
               ADV_CUDA(adv::launch_basis_change(n, u, ch.cell(ch.z[c]), ch.cell(ch.z[c + 1]), true, s, tr_basis,
-                                                trace_width(*h), tr_upwind));
+                                                trace_width(*h), tr_upwind, fixed));
               ++h->launches;
             }
           for (int l = ch.z[c]; l < ch.z[c + 1]; ++l)
@@ -1339,7 +1340,7 @@ int run_steps(adv_handle *h, int n_steps, int ns, bool gauss, bool traces, doubl
     }
   else if (gauss)
     {
-      ADV_CUDA(adv::launch_basis_change(n, u, cb, ce, true, s, tr_basis, trace_width(*h), tr_upwind));
+      ADV_CUDA(adv::launch_basis_change(n, u, cb, ce, true, s, tr_basis, trace_width(*h), tr_upwind, fixed));
       ++h->launches;
     }
   for (int step = 0; step < n_steps; ++step)
@@ -1366,7 +1367,8 @@ int run_steps(adv_handle *h, int n_steps, int ns, bool gauss, bool traces, doubl
               return e;
             if (gauss)
               {
-                ADV_CUDA(adv::launch_basis_change(n, u, ch.cell(ch.z[c]), ch.cell(ch.z[c + 1]), false, s));
+                ADV_CUDA(adv::launch_basis_change(n, u, ch.cell(ch.z[c]), ch.cell(ch.z[c + 1]), false, s, nullptr, 1, nullptr,
+                                                      fixed));
                 ++h->launches;
               }
             const int64_t d0 = ch.dof(ch.z[c]), d1 = ch.dof(ch.z[c + 1]);
@@ -1379,7 +1381,7 @@ int run_steps(adv_handle *h, int n_steps, int ns, bool gauss, bool traces, doubl
       }
   if (gauss && !host)
     {
-      ADV_CUDA(adv::launch_basis_change(n, u, cb, ce, false, s));
+      ADV_CUDA(adv::launch_basis_change(n, u, cb, ce, false, s, nullptr, 1, nullptr, fixed));
       ++h->launches;
     }
   return ADV_OK;

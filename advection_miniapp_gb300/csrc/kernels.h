@@ -132,9 +132,10 @@ cudaError_t upload_tables_gauss32(const DevTables<double> *d, const DevTables<fl
 // (width 1): only the traces an upwind-trace stage reads (StageArgs::
 // upwind_tr), with the mesh and the FP64 face coefficients of *upwind; (width
 // 2) traces as the block fixed-point stages form them (upwind->fx_visc).
+// fixed: block fixed-point sweeps, else binary64 (the FP32 operator).
 cudaError_t launch_basis_change(int n, double *u, long long cell_begin, long long cell_end, bool to_gauss,
                                 cudaStream_t stream, double *traces = nullptr, int width = 1,
-                                const StageArgs *upwind = nullptr);
+                                const StageArgs *upwind = nullptr, bool fixed = true);
 // In-place u <- (S^T x S^T x S^T) u for the cells [cell_begin, cell_end): the
 // dual coefficients of a weak-form vector on the Gauss-point basis to those
 // on the Gauss-Lobatto nodal basis (each nodal function is the combination

@@ -18,13 +18,15 @@ namespace
 // kernel writes them.
 // The sweeps run in block fixed point, one power of two per cell (fixed.cuh);
 // a cell outside the window of exponents (infinities, NaN, magnitudes outside
-// 2^-400 .. 2^600) in binary64.  The shared buffer holds binary64 values or
+// 2^-400 .. 2^600) in binary64, and all cells without `fixed` (the FP32
+// operator, whose solutions a change in the last bit of its input changes by their
+// own round-off).  The shared buffer holds binary64 values or
 // limbs, 8 bytes each.  Measured on GB300 at 48^3 cells of degree 4 (a step
 // through host memory, with both changes of basis in 8 chunks): 2.53 instead
 // of 2.84 ms with binary64 sweeps (79 % of the FP64 peak).
 template <int N, int MODE, bool UPW>
 __global__ void __launch_bounds__(StageShape<N, double, true, false>::THREADS)
-  basis_kernel(double *u, long long cell_begin, long long cell_end, double *traces, int width,
+  basis_kernel(double *u, long long cell_begin, long long cell_end, double *traces, int width, bool fixed,
                const __grid_constant__ StageArgs F)
 {
   using SH         = StageShape<N, double, true, false>;
@@ -86,7 +88,7 @@ __global__ void __launch_bounds__(StageShape<N, double, true, false>::THREADS)
         }
       __syncthreads();
       int        top  = 1023;
-      const bool live = mine && fx_window(s_max[cl], top);
+      const bool live = mine && fx_window(s_max[cl], top) && fixed;
       int2      *lb   = reinterpret_cast<int2 *>(buf);
       // a sweep in binary64, of a cell outside the window
       auto sweep64 = [&](double *p, int st, double(&out)[N]) {
@@ -220,7 +222,7 @@ __global__ void __launch_bounds__(StageShape<N, double, true, false>::THREADS)
 
 template <int N>
 cudaError_t launch_basis_n(double *u, long long cell_begin, long long cell_end, int mode, cudaStream_t s,
-                           double *traces, int width, const StageArgs *upwind)
+                           double *traces, int width, const StageArgs *upwind, bool fixed)
 {
   using SH               = StageShape<N, double, true, false>;
   const long long blocks = (cell_end - cell_begin + SH::C - 1) / SH::C;
@@ -233,17 +235,17 @@ cudaError_t launch_basis_n(double *u, long long cell_begin, long long cell_end, 
     memset(&F, 0, sizeof(F));
   const bool upw = upwind && traces && width == 1;
   if (mode == 1 && upw)
-    basis_kernel<N, 1, true><<<(unsigned)blocks, SH::THREADS, 0, s>>>(u, cell_begin, cell_end, traces, width, F);
+    basis_kernel<N, 1, true><<<(unsigned)blocks, SH::THREADS, 0, s>>>(u, cell_begin, cell_end, traces, width, fixed, F);
   else if (mode == 1)
-    basis_kernel<N, 1, false><<<(unsigned)blocks, SH::THREADS, 0, s>>>(u, cell_begin, cell_end, traces, width, F);
+    basis_kernel<N, 1, false><<<(unsigned)blocks, SH::THREADS, 0, s>>>(u, cell_begin, cell_end, traces, width, fixed, F);
   else if (mode == 2 && upw)
-    basis_kernel<N, 2, true><<<(unsigned)blocks, SH::THREADS, 0, s>>>(u, cell_begin, cell_end, traces, width, F);
+    basis_kernel<N, 2, true><<<(unsigned)blocks, SH::THREADS, 0, s>>>(u, cell_begin, cell_end, traces, width, fixed, F);
   else if (mode == 2)
-    basis_kernel<N, 2, false><<<(unsigned)blocks, SH::THREADS, 0, s>>>(u, cell_begin, cell_end, traces, width, F);
+    basis_kernel<N, 2, false><<<(unsigned)blocks, SH::THREADS, 0, s>>>(u, cell_begin, cell_end, traces, width, fixed, F);
   else if (mode == 3)
-    basis_kernel<N, 3, false><<<(unsigned)blocks, SH::THREADS, 0, s>>>(u, cell_begin, cell_end, nullptr, 1, F);
+    basis_kernel<N, 3, false><<<(unsigned)blocks, SH::THREADS, 0, s>>>(u, cell_begin, cell_end, nullptr, 1, fixed, F);
   else
-    basis_kernel<N, 0, false><<<(unsigned)blocks, SH::THREADS, 0, s>>>(u, cell_begin, cell_end, nullptr, 1, F);
+    basis_kernel<N, 0, false><<<(unsigned)blocks, SH::THREADS, 0, s>>>(u, cell_begin, cell_end, nullptr, 1, fixed, F);
   return cudaGetLastError();
 }
 } // namespace
@@ -272,25 +274,26 @@ cudaError_t launch_stage_gauss_fp64(int n, const StageArgs &args, cudaStream_t s
 namespace
 {
 cudaError_t launch_basis_mode(int n, double *u, long long cell_begin, long long cell_end, int mode,
-                              cudaStream_t stream, double *traces, int width, const StageArgs *upwind = nullptr)
+                              cudaStream_t stream, double *traces, int width, const StageArgs *upwind = nullptr,
+                              bool fixed = true)
 {
   switch (n)
     {
-      case 2: return launch_basis_n<2>(u, cell_begin, cell_end, mode, stream, traces, width, upwind);
-      case 3: return launch_basis_n<3>(u, cell_begin, cell_end, mode, stream, traces, width, upwind);
-      case 4: return launch_basis_n<4>(u, cell_begin, cell_end, mode, stream, traces, width, upwind);
-      case 5: return launch_basis_n<5>(u, cell_begin, cell_end, mode, stream, traces, width, upwind);
-      case 6: return launch_basis_n<6>(u, cell_begin, cell_end, mode, stream, traces, width, upwind);
-      case 7: return launch_basis_n<7>(u, cell_begin, cell_end, mode, stream, traces, width, upwind);
+      case 2: return launch_basis_n<2>(u, cell_begin, cell_end, mode, stream, traces, width, upwind, fixed);
+      case 3: return launch_basis_n<3>(u, cell_begin, cell_end, mode, stream, traces, width, upwind, fixed);
+      case 4: return launch_basis_n<4>(u, cell_begin, cell_end, mode, stream, traces, width, upwind, fixed);
+      case 5: return launch_basis_n<5>(u, cell_begin, cell_end, mode, stream, traces, width, upwind, fixed);
+      case 6: return launch_basis_n<6>(u, cell_begin, cell_end, mode, stream, traces, width, upwind, fixed);
+      case 7: return launch_basis_n<7>(u, cell_begin, cell_end, mode, stream, traces, width, upwind, fixed);
       default: return cudaErrorInvalidValue;
     }
 }
 } // namespace
 
 cudaError_t launch_basis_change(int n, double *u, long long cell_begin, long long cell_end, bool to_gauss,
-                                cudaStream_t stream, double *traces, int width, const StageArgs *upwind)
+                                cudaStream_t stream, double *traces, int width, const StageArgs *upwind, bool fixed)
 {
-  return launch_basis_mode(n, u, cell_begin, cell_end, to_gauss ? 1 : 0, stream, traces, width, upwind);
+  return launch_basis_mode(n, u, cell_begin, cell_end, to_gauss ? 1 : 0, stream, traces, width, upwind, fixed);
 }
 
 cudaError_t launch_basis_dual_to_nodal(int n, double *u, long long cell_begin, long long cell_end,
