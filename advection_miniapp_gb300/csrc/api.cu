@@ -367,7 +367,6 @@ adv::StageArgs base_args(const adv_handle &h, double t, int prec = -1)
   A.cell_geo = geo64 ? (const void *)h.d_cell_geo64 : h.d_cell_geo;
   A.fx_ok    = h.fx_ok;
   A.cell_exp = h.d_cell_exp;
-  A.vt_limbs = h.fx_ok;
   A.fx_visc  = h.fx_visc;
   A.t        = t;
   A.ex       = h.diag.ex;
@@ -628,8 +627,11 @@ int create_handle(const adv_config *cfg, int z_begin, int z_end, adv_handle **ou
         h->cv[d] = g.cv[d], h->P[d] = g.P[d], h->M[d] = g.M[d];
       const bool fp64 = h->cfg.precision == ADV_PRECISION_FP64;
       const bool both = h->cfg.precision == ADV_PRECISION_FP32_INCREMENT;
-      // the block fixed-point stages: every form with an FP64 operator
-      h->fx_ok = g.fx_ok && (fp64 || both) && h->cfg.diffusion == 0.0 && h->cfg.factor_skew == 0.0;
+      // the block fixed-point stages: the FP64 operator.  (The FP32 increments'
+      // FP64 anchor stays binary64: a change in the last bit of K0 or of the
+      // Gauss-point values turns single binary32 roundings, which the stages
+      // spread, and the solution moves by up to 4e-8 of its size.)
+      h->fx_ok = g.fx_ok && fp64 && h->cfg.diffusion == 0.0 && h->cfg.factor_skew == 0.0;
       h->fx_visc = g.fx_ok && fp64 && h->cfg.diffusion != 0.0 && h->cfg.factor_skew == 0.0 &&
                    sipg_in_fx_window(h->cfg, h->mesh);
       if ((h->fx_ok || h->fx_visc) && !g.cell_exp.empty())
@@ -649,8 +651,6 @@ int create_handle(const adv_config *cfg, int z_begin, int z_end, adv_handle **ou
             vt_to_limbs(h->mesh, g);
           rc = fp64 ? upload_array<double>(g.cell, &h->d_cell_geo, h->device_bytes)
                     : upload_array<float>(g.cell, &h->d_cell_geo, h->device_bytes);
-          if (both && h->fx_ok)
-            vt_to_limbs(h->mesh, g);
           if (rc == ADV_OK && both)
             rc = upload_array<double>(g.cell, (void **)&h->d_cell_geo64, h->device_bytes);
         }
@@ -1261,7 +1261,7 @@ int run_steps(adv_handle *h, int n_steps, int ns, bool gauss, bool traces, doubl
   if (tr_args)
     upw = base_args(*h, 0.0, 0);
   const adv::StageArgs *tr_upwind = tr_args ? &upw : nullptr;
-  const bool            fixed     = h->cfg.precision != ADV_PRECISION_FP32_OPERATOR;
+  const bool            fixed     = h->cfg.precision == ADV_PRECISION_FP64;
   HostChunks    ch;
   int           nch = 0;
   if (host)

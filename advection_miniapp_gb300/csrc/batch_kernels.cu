@@ -91,9 +91,9 @@ __global__ void __launch_bounds__(StageShape<N, T, true, false>::THREADS) batch_
   if constexpr (kBatchCollocation<T>)
     {
       if (sA.fx_ok)
-        stage_fx_cta<N, true, true, false, false>(sA, cell0, smem_raw);
+        stage_fx_cta<N, true, true, false>(sA, cell0, smem_raw);
       else
-        stage_gauss_masked<N, true, true, false, false>(sA, cell0, smem_raw, ~0u);
+        stage_gauss_masked<N, true, true, false>(sA, cell0, smem_raw, ~0u);
     }
   else
     stage_cta<N, T, true, false>(sA, cell0, smem_raw);

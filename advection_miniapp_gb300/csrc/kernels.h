@@ -60,9 +60,9 @@ struct StageArgs
   // block fixed-point path (stage_fx.cuh): allowed for this mesh (vt, 1 / det J
   // or the uniform constants within 2^+-200), and in the field case the
   // largest biased binary64 exponent of vt per cell
+  // (vt of cell_geo is then stored as limbs, fx_const58 with the cell's exponent)
   int           fx_ok;
   int           fx_visc;  // the same for the diffusive stages (vt stays binary64 there)
-  int           vt_limbs; // field case: vt of cell_geo as limbs (fx_const58 with the cell's exponent)
   const int    *cell_exp;
   const void   *cell_geo;    // field case: [vt0|vt1|vt2|idet] x n^3 per cell (T)
   const void   *face_geo[3]; // field case: n^2 (P, M) pairs per face (T)
@@ -132,7 +132,7 @@ cudaError_t upload_tables_gauss32(const DevTables<double> *d, const DevTables<fl
 // (width 1): only the traces an upwind-trace stage reads (StageArgs::
 // upwind_tr), with the mesh and the FP64 face coefficients of *upwind; (width
 // 2) traces as the block fixed-point stages form them (upwind->fx_visc).
-// fixed: block fixed-point sweeps, else binary64 (the FP32 operator).
+// fixed: block fixed-point sweeps, else binary64 (the FP32 operator and increments).
 cudaError_t launch_basis_change(int n, double *u, long long cell_begin, long long cell_end, bool to_gauss,
                                 cudaStream_t stream, double *traces = nullptr, int width = 1,
                                 const StageArgs *upwind = nullptr, bool fixed = true);

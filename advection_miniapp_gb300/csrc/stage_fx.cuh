@@ -48,11 +48,11 @@ struct FxShape
 };
 
 // the binary64 path for the cells of `mask`
-template <int N, bool UNI, bool TR, bool INC, bool UPW>
+template <int N, bool UNI, bool TR, bool UPW>
 __device__ __noinline__ void stage_gauss_masked(const StageArgs &A, long long cell0, unsigned char *smem,
                                                 unsigned mask)
 {
-  stage_gauss_cta<N, double, UNI, false, TR, INC, UPW>(A, cell0, smem, mask);
+  stage_gauss_cta<N, double, UNI, false, TR, false, UPW, !UNI>(A, cell0, smem, mask);
 }
 
 // The traces of a pencil x that the next stage reads: at the low face if bit 0
@@ -84,7 +84,7 @@ static __device__ __noinline__ double boundary_value(const StageArgs &A, int d, 
   return exact_value(A.ex, x[0], x[1], x[2], A.t);
 }
 
-template <int N, bool UNI, bool TR, bool INC, bool UPW>
+template <int N, bool UNI, bool TR, bool UPW>
 __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long cell0, unsigned char *smem_raw)
 {
   using FS         = FxShape<N, UNI, TR>;
@@ -310,7 +310,7 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
     }
   // the update's read of the solution ahead of the last pass
   const long long gb        = (cell0 + cl) * NQ + r;
-  const bool      reads_u   = !INC && (A.mode == kModeStage || A.mode == kModeLastStage) && (TR || A.u_in);
+  const bool      reads_u   = (A.mode == kModeStage || A.mode == kModeLastStage) && (TR || A.u_in);
   double          ui[N];
 #pragma unroll
   for (int k = 0; k < N; ++k)
@@ -328,7 +328,7 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
 #pragma unroll
       for (int k = 0; k < N; ++k)
         kd[k] = fx_to_double(Qb[off + k * NF] + out[k], ez);
-      if (!TR && !INC && A.mode == kModeVmult)
+      if (!TR && A.mode == kModeVmult)
         {
           // implicit operator in weak form: JxW (c U - bracket), as stage_gauss_cta
 #pragma unroll
@@ -348,18 +348,7 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
               for (int k = 0; k < N; ++k)
                 kd[k] *= G[3 * NQ + r + k * NF];
             }
-          if (INC)
-            {
-              // the FP32 increments' FP64 anchor: K0 and the first G
-#pragma unroll
-              for (int k = 0; k < N; ++k)
-                {
-                  A.k_out[gb + k * NF]   = kd[k];
-                  A.k_out32[gb + k * NF] = d2f_int(kd[k]);
-                  A.r_out32[gb + k * NF] = d2f_int(A.a * kd[k]);
-                }
-            }
-          else if (A.mode == kModeApply)
+          if (A.mode == kModeApply)
             {
 #pragma unroll
               for (int k = 0; k < N; ++k)
@@ -402,7 +391,7 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
                 }
             }
         }
-      if (TR && !INC && A.tr_out)
+      if (TR && A.tr_out)
         {
           write_traces<N>(tb, next, own >> 4, static_cast<double *>(A.tr_out) + ((cell0 + cl) * 6 + 4) * NF + r);
 #pragma unroll
@@ -410,7 +399,7 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
             Qb[off + k * NF] = __double_as_longlong(next[k]);
         }
     }
-  if (TR && !INC && A.tr_out)
+  if (TR && A.tr_out)
     {
       __syncthreads();
       if (live)
@@ -434,23 +423,23 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
   if (bad)
     {
       __syncthreads();
-      stage_gauss_masked<N, UNI, TR, INC, UPW>(A, cell0, smem_raw, bad);
+      stage_gauss_masked<N, UNI, TR, UPW>(A, cell0, smem_raw, bad);
     }
 }
 
-template <int N, bool UNI, bool TR, bool INC, bool UPW>
+template <int N, bool UNI, bool TR, bool UPW>
 __global__ void __launch_bounds__(FxShape<N, UNI, TR>::THREADS, kFxThreadsPerSM / FxShape<N, UNI, TR>::THREADS)
   stage_fx_kernel(const __grid_constant__ StageArgs A)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  stage_fx_cta<N, UNI, TR, INC, UPW>(A, A.cell_begin + (long long)blockIdx.x * FxShape<N, UNI, TR>::C, smem_raw);
+  stage_fx_cta<N, UNI, TR, UPW>(A, A.cell_begin + (long long)blockIdx.x * FxShape<N, UNI, TR>::C, smem_raw);
 }
 
-template <int N, bool UNI, bool TR, bool INC = false, bool UPW = false>
+template <int N, bool UNI, bool TR, bool UPW = false>
 cudaError_t launch_stage_fx_t(const StageArgs &args, cudaStream_t stream)
 {
   using FS              = FxShape<N, UNI, TR>;
-  constexpr auto kernel = stage_fx_kernel<N, UNI, TR, INC, UPW>;
+  constexpr auto kernel = stage_fx_kernel<N, UNI, TR, UPW>;
   static std::atomic<unsigned long long> configured{0};
   cudaError_t                            e = opt_in_smem(kernel, FS::SMEM, configured);
   if (e != cudaSuccess)
@@ -466,18 +455,9 @@ template <int N>
 cudaError_t launch_stage_fx_n(const StageArgs &args, cudaStream_t stream)
 {
   if (args.tr_in)
-    {
-      if (args.uniform)
-        return launch_stage_fx_t<N, true, true>(args, stream);
-      if (args.inc32)
-        return args.upwind_tr ? launch_stage_fx_t<N, false, true, true, true>(args, stream)
-                              : launch_stage_fx_t<N, false, true, true>(args, stream);
-      return args.upwind_tr ? launch_stage_fx_t<N, false, true, false, true>(args, stream)
+    return args.uniform     ? launch_stage_fx_t<N, true, true>(args, stream)
+           : args.upwind_tr ? launch_stage_fx_t<N, false, true, true>(args, stream)
                             : launch_stage_fx_t<N, false, true>(args, stream);
-    }
-  if (args.inc32)
-    return args.uniform ? launch_stage_fx_t<N, true, false, true>(args, stream)
-                        : launch_stage_fx_t<N, false, false, true>(args, stream);
   return args.uniform ? launch_stage_fx_t<N, true, false>(args, stream)
                       : launch_stage_fx_t<N, false, false>(args, stream);
 }

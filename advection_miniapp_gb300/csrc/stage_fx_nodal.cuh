@@ -42,7 +42,7 @@ struct FxNodalShape
 template <int N, bool UNI>
 __device__ __noinline__ void stage_nodal_masked(const StageArgs &A, long long cell0, unsigned char *smem, unsigned mask)
 {
-  stage_cta<N, double, UNI, false>(A, cell0, smem, mask);
+  stage_cta<N, double, UNI, false, !UNI>(A, cell0, smem, mask);
 }
 
 template <int N, bool UNI>

@@ -131,7 +131,8 @@ __device__ __forceinline__ bool upwind_pencil_traces(const DevTables<T> &tb, con
 // increment form's.  FP64 operator: the block's anchor (writes K0 and the
 // first G).
 // cell_mask: the cells of the CTA (bit cl) whose outputs are written.
-template <int N, typename T, bool UNI, bool VISC, bool TR = false, bool INC = false, bool UPW = false>
+template <int N, typename T, bool UNI, bool VISC, bool TR = false, bool INC = false, bool UPW = false,
+          bool LIMBS = false>
 __device__ __forceinline__ void stage_gauss_cta(const StageArgs &A, const long long cell0,
                                                 unsigned char *smem_raw, unsigned cell_mask = ~0u)
 {
@@ -419,17 +420,17 @@ __device__ __forceinline__ void stage_gauss_cta(const StageArgs &A, const long l
           upwind_values(cl, 0, r, pm, vlo, vhi, own_lo, own_hi);
           s_need[(cl * 6 + 0) * NF + r] = own_lo;
           s_need[(cl * 6 + 1) * NF + r] = own_hi;
-          direction_pass_pm<N, T, UNI, VISC, 0, true, true>(A, tb, U, vlo, vhi, T(0), T(0), false, false, pm,
+          direction_pass_pm<N, T, UNI, VISC, 0, true, true, LIMBS>(A, tb, U, vlo, vhi, T(0), T(0), false, false, pm,
                                                             geo(cl) + N * r, 1, out, T(0), T(0), T(0), T(0),
-                                                            vt_top(A, cell0 + cl));
+                                                            vt_top<LIMBS>(A, cell0 + cl));
         }
       else
-        direction_pass<N, T, UNI, VISC, 0, TR>(A, tb, U, nbv(cl, 0, r), nbv(cl, 1, r), nbd(cl, 0, r),
+        direction_pass<N, T, UNI, VISC, 0, TR, LIMBS>(A, tb, U, nbv(cl, 0, r), nbv(cl, 1, r), nbd(cl, 0, r),
                                                nbd(cl, 1, r), s_nbr[cl * 6 + 0] < 0, s_nbr[cl * 6 + 1] < 0, r,
                                                faces(cl, 0), faces(cl, 1), geo(cl) + N * r, 1, out,
                                                TR ? trv(Tr, 0) : T(0), TR ? trv(Tr, TRW * NF) : T(0),
                                                TR && VISC ? trv(Tr, NF) : T(0),
-                                               TR && VISC ? trv(Tr, TRW * NF + NF) : T(0), vt_top(A, cell0 + cl));
+                                               TR && VISC ? trv(Tr, TRW * NF + NF) : T(0), vt_top<LIMBS>(A, cell0 + cl));
       T *z = Qb + cl * NQ + N * r;
 #pragma unroll
       for (int k = 0; k < N; ++k)
@@ -456,17 +457,17 @@ __device__ __forceinline__ void stage_gauss_cta(const StageArgs &A, const long l
           upwind_values(cl, 2, r, pm, vlo, vhi, own_lo, own_hi);
           s_need[(cl * 6 + 2) * NF + r] = own_lo;
           s_need[(cl * 6 + 3) * NF + r] = own_hi;
-          direction_pass_pm<N, T, UNI, VISC, 1, true, true>(A, tb, U, vlo, vhi, T(0), T(0), false, false, pm,
+          direction_pass_pm<N, T, UNI, VISC, 1, true, true, LIMBS>(A, tb, U, vlo, vhi, T(0), T(0), false, false, pm,
                                                             geo(cl) + NQ + off, N, out, T(0), T(0), T(0), T(0),
-                                                            vt_top(A, cell0 + cl));
+                                                            vt_top<LIMBS>(A, cell0 + cl));
         }
       else
-        direction_pass<N, T, UNI, VISC, 1, TR>(A, tb, U, nbv(cl, 2, r), nbv(cl, 3, r), nbd(cl, 2, r),
+        direction_pass<N, T, UNI, VISC, 1, TR, LIMBS>(A, tb, U, nbv(cl, 2, r), nbv(cl, 3, r), nbd(cl, 2, r),
                                                nbd(cl, 3, r), s_nbr[cl * 6 + 2] < 0, s_nbr[cl * 6 + 3] < 0, r,
                                                faces(cl, 2), faces(cl, 3), geo(cl) + NQ + off, N, out,
                                                TR ? trv(Tr, 0) : T(0), TR ? trv(Tr, TRW * NF) : T(0),
                                                TR && VISC ? trv(Tr, NF) : T(0),
-                                               TR && VISC ? trv(Tr, TRW * NF + NF) : T(0), vt_top(A, cell0 + cl));
+                                               TR && VISC ? trv(Tr, TRW * NF + NF) : T(0), vt_top<LIMBS>(A, cell0 + cl));
       T *z = Qb + cl * NQ + off;
 #pragma unroll
       for (int k = 0; k < N; ++k)
@@ -494,17 +495,17 @@ __device__ __forceinline__ void stage_gauss_cta(const StageArgs &A, const long l
           FacePM<T> pm;
           T         vlo, vhi;
           upwind_values(cl, 4, r, pm, vlo, vhi, zlo, zhi);
-          direction_pass_pm<N, T, UNI, VISC, 2, true, true>(A, tb, U, vlo, vhi, T(0), T(0), false, false, pm,
+          direction_pass_pm<N, T, UNI, VISC, 2, true, true, LIMBS>(A, tb, U, vlo, vhi, T(0), T(0), false, false, pm,
                                                             G + 2 * NQ + r, NF, out, T(0), T(0), T(0), T(0),
-                                                            vt_top(A, cell0 + cl));
+                                                            vt_top<LIMBS>(A, cell0 + cl));
         }
       else
-        direction_pass<N, T, UNI, VISC, 2, TR>(A, tb, U, nbv(cl, 4, r), nbv(cl, 5, r), nbd(cl, 4, r),
+        direction_pass<N, T, UNI, VISC, 2, TR, LIMBS>(A, tb, U, nbv(cl, 4, r), nbv(cl, 5, r), nbd(cl, 4, r),
                                                nbd(cl, 5, r), s_nbr[cl * 6 + 4] < 0, s_nbr[cl * 6 + 5] < 0, r,
                                                faces(cl, 4), faces(cl, 5), G + 2 * NQ + r, NF, out,
                                                TR ? trv(Tr, 0) : T(0), TR ? trv(Tr, TRW * NF) : T(0),
                                                TR && VISC ? trv(Tr, NF) : T(0),
-                                               TR && VISC ? trv(Tr, TRW * NF + NF) : T(0), vt_top(A, cell0 + cl));
+                                               TR && VISC ? trv(Tr, TRW * NF + NF) : T(0), vt_top<LIMBS>(A, cell0 + cl));
       T              *z  = Qb + cl * NQ + r;
       const long long gb = (cell0 + cl) * NQ + r;
       double          next[N]; // the next stage's input along the pencil (traces)

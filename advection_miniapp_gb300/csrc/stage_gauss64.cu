@@ -18,15 +18,13 @@ namespace
 // kernel writes them.
 // The sweeps run in block fixed point, one power of two per cell (fixed.cuh);
 // a cell outside the window of exponents (infinities, NaN, magnitudes outside
-// 2^-400 .. 2^600) in binary64, and all cells without `fixed` (the FP32
-// operator, whose solutions a change in the last bit of its input changes by their
-// own round-off).  The shared buffer holds binary64 values or
+// 2^-400 .. 2^600) in binary64.  The shared buffer holds binary64 values or
 // limbs, 8 bytes each.  Measured on GB300 at 48^3 cells of degree 4 (a step
 // through host memory, with both changes of basis in 8 chunks): 2.53 instead
 // of 2.84 ms with binary64 sweeps (79 % of the FP64 peak).
 template <int N, int MODE, bool UPW>
 __global__ void __launch_bounds__(StageShape<N, double, true, false>::THREADS)
-  basis_kernel(double *u, long long cell_begin, long long cell_end, double *traces, int width, bool fixed,
+  basis_kernel(double *u, long long cell_begin, long long cell_end, double *traces, int width,
                const __grid_constant__ StageArgs F)
 {
   using SH         = StageShape<N, double, true, false>;
@@ -88,7 +86,7 @@ __global__ void __launch_bounds__(StageShape<N, double, true, false>::THREADS)
         }
       __syncthreads();
       int        top  = 1023;
-      const bool live = mine && fx_window(s_max[cl], top) && fixed;
+      const bool live = mine && fx_window(s_max[cl], top);
       int2      *lb   = reinterpret_cast<int2 *>(buf);
       // a sweep in binary64, of a cell outside the window
       auto sweep64 = [&](double *p, int st, double(&out)[N]) {
@@ -220,6 +218,119 @@ __global__ void __launch_bounds__(StageShape<N, double, true, false>::THREADS)
     }
 }
 
+// The same in binary64 (modes 0 and 1), for the FP32 operator and increments:
+// a change in the last bit of their input turns single binary32 roundings,
+// which the stages spread, so their solutions would move by their own round-off.
+template <int N, int MODE, bool UPW>
+__global__ void __launch_bounds__(StageShape<N, double, true, false>::THREADS)
+  basis64_kernel(double *u, long long cell_begin, long long cell_end, double *traces, int width, const StageArgs F)
+{
+  using SH         = StageShape<N, double, true, false>;
+  constexpr int C  = SH::C;
+  constexpr int NQ = SH::NQ;
+  constexpr int NF = SH::NF;
+  constexpr int NT = SH::THREADS;
+  __shared__ double    buf[C * NQ];
+  // upwind traces: face ids, and the pencils whose high trace is deferred
+  __shared__ int           s_face[UPW ? 6 * C : 1], s_nbr[UPW ? 6 * C : 1], s_nboth, s_both[UPW ? 3 * C * NF : 1];
+  const DevTables<double> &tb    = tab<double>(N);
+  const long long          cell0 = cell_begin + (long long)blockIdx.x * C;
+  const int                ncell = (int)min((long long)C, cell_end - cell0);
+  const int                tid   = threadIdx.x;
+  double                  *g     = u + cell0 * NQ;
+  constexpr bool TO_GAUSS = MODE == 1;
+  if (UPW)
+    {
+      cell_neighbours(F, cell0, ncell, s_nbr, s_face, tid, NT);
+      if (tid == 0)
+        s_nboth = 0;
+    }
+  for (int i = tid; i < ncell * NQ; i += NT)
+    buf[i] = g[i];
+  __syncthreads();
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+    {
+      for (int w = tid; w < ncell * NF; w += NT)
+        {
+          const int cl = w / NF, r = w % NF;
+          const int off = d == 0 ? N * r : d == 1 ? (r % N) + NF * (r / N) : r;
+          const int st  = d == 0 ? 1 : d == 1 ? N : NF;
+          double   *p   = buf + cl * NQ + off;
+          double    in[N], out[N];
+#pragma unroll
+          for (int k = 0; k < N; ++k)
+            in[k] = p[k * st];
+          if (TO_GAUSS)
+            sweep2<N, double, false>(tb.S, tb.S_eo, in, out);
+          else
+            sweep2<N, double, false>(tb.Si, tb.Si_eo, in, out);
+#pragma unroll
+          for (int k = 0; k < N; ++k)
+            p[k * st] = out[k];
+        }
+      __syncthreads();
+    }
+  for (int i = tid; i < ncell * NQ; i += NT)
+    g[i] = buf[i];
+  if (MODE != 0 && traces)
+    {
+      // face traces of the result, [6][width][NF] per cell (StageArgs::tr_in):
+      // values, and with width 2 also reference normal derivatives
+      for (int w = tid; w < 3 * ncell * NF; w += NT)
+        {
+          const int d = w / (ncell * NF), v = w % (ncell * NF);
+          const int cl = v / NF, r = v % NF;
+          const int off = d == 0 ? N * r : d == 1 ? (r % N) + NF * (r / N) : r;
+          const int st  = d == 0 ? 1 : d == 1 ? N : NF;
+          double    x[N], lo, hi;
+#pragma unroll
+          for (int k = 0; k < N; ++k)
+            x[k] = buf[cl * NQ + off + k * st];
+          double *to = traces + ((cell0 + cl) * 6 + 2 * d) * width * NF + r;
+          if (UPW)
+            {
+              // own trace read on the low face where M != 0, on the high face where P != 0
+              const double *fg = d == 0 ? static_cast<const double *>(F.face_geo[0])
+                               : d == 1 ? static_cast<const double *>(F.face_geo[1])
+                                        : static_cast<const double *>(F.face_geo[2]);
+              const double2 pl = *reinterpret_cast<const double2 *>(fg + (size_t)s_face[cl * 6 + 2 * d] * 2 * NF + 2 * r);
+              const double2 ph =
+                *reinterpret_cast<const double2 *>(fg + (size_t)s_face[cl * 6 + 2 * d + 1] * 2 * NF + 2 * r);
+              if (upwind_pencil_traces<N, double>(tb, x, nonzero(pl.y), nonzero(ph.x), to, to + NF))
+                s_both[atomicAdd(&s_nboth, 1)] = (d * C + cl) * NF + r;
+              continue;
+            }
+          pencil_traces<N, double>(tb, x, lo, hi);
+          to[0]          = lo;
+          to[width * NF] = hi;
+          if (width == 2)
+            {
+              pencil_dtraces<N, double>(tb, x, lo, hi);
+              to[NF]     = lo;
+              to[3 * NF] = hi;
+            }
+        }
+      if (UPW)
+        {
+          // the deferred high traces (usually none)
+          __syncthreads();
+          for (int i = tid; i < s_nboth; i += NT)
+            {
+              const int code = s_both[i];
+              const int d = code / (C * NF), cl = (code / NF) % C, r = code % NF;
+              const int off = d == 0 ? N * r : d == 1 ? (r % N) + NF * (r / N) : r;
+              const int st  = d == 0 ? 1 : d == 1 ? N : NF;
+              double    h   = tb.l1[0] * buf[cl * NQ + off];
+#pragma unroll
+              for (int q = 1; q < N; ++q)
+                h = fma(tb.l1[q], buf[cl * NQ + off + q * st], h);
+              traces[((cell0 + cl) * 6 + 2 * d + 1) * NF + r] = h;
+            }
+        }
+    }
+}
+
 template <int N>
 cudaError_t launch_basis_n(double *u, long long cell_begin, long long cell_end, int mode, cudaStream_t s,
                            double *traces, int width, const StageArgs *upwind, bool fixed)
@@ -233,19 +344,22 @@ cudaError_t launch_basis_n(double *u, long long cell_begin, long long cell_end, 
     F = *upwind;
   else
     memset(&F, 0, sizeof(F));
-  const bool upw = upwind && traces && width == 1;
+  const bool upw  = upwind && traces && width == 1;
+  auto       call = [&](auto kernel, double *tr, int w) {
+    kernel<<<(unsigned)blocks, SH::THREADS, 0, s>>>(u, cell_begin, cell_end, tr, w, F);
+  };
   if (mode == 1 && upw)
-    basis_kernel<N, 1, true><<<(unsigned)blocks, SH::THREADS, 0, s>>>(u, cell_begin, cell_end, traces, width, fixed, F);
+    call(fixed ? basis_kernel<N, 1, true> : basis64_kernel<N, 1, true>, traces, width);
   else if (mode == 1)
-    basis_kernel<N, 1, false><<<(unsigned)blocks, SH::THREADS, 0, s>>>(u, cell_begin, cell_end, traces, width, fixed, F);
+    call(fixed ? basis_kernel<N, 1, false> : basis64_kernel<N, 1, false>, traces, width);
   else if (mode == 2 && upw)
-    basis_kernel<N, 2, true><<<(unsigned)blocks, SH::THREADS, 0, s>>>(u, cell_begin, cell_end, traces, width, fixed, F);
+    call(basis_kernel<N, 2, true>, traces, width);
   else if (mode == 2)
-    basis_kernel<N, 2, false><<<(unsigned)blocks, SH::THREADS, 0, s>>>(u, cell_begin, cell_end, traces, width, fixed, F);
+    call(basis_kernel<N, 2, false>, traces, width);
   else if (mode == 3)
-    basis_kernel<N, 3, false><<<(unsigned)blocks, SH::THREADS, 0, s>>>(u, cell_begin, cell_end, nullptr, 1, fixed, F);
+    call(basis_kernel<N, 3, false>, nullptr, 1);
   else
-    basis_kernel<N, 0, false><<<(unsigned)blocks, SH::THREADS, 0, s>>>(u, cell_begin, cell_end, nullptr, 1, fixed, F);
+    call(fixed ? basis_kernel<N, 0, false> : basis64_kernel<N, 0, false>, nullptr, 1);
   return cudaGetLastError();
 }
 } // namespace

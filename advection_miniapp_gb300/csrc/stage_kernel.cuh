@@ -316,12 +316,17 @@ __device__ __forceinline__ FacePM<T> face_pm(const StageArgs &A, const T *Flo, c
 // value on the upwind side there, own or neighbour; the flux is then one
 // product per face, with the same value as the general form.
 // exponent of a cell's vt limbs
+template <bool LIMBS>
 __device__ __forceinline__ int vt_top(const StageArgs &A, long long c)
 {
-  return A.vt_limbs ? A.cell_exp[c] : 0;
+  return LIMBS ? A.cell_exp[c] : 0;
 }
 
-template <int N, typename T, bool UNI, bool VISC, int D, bool OWN_TR = false, bool UPW = false>
+// LIMBS: vt as limbs with the cell's exponent vtop (the cell geometry of the
+// block fixed-point kernels, whose cells outside their window run here); a
+// compile-time variant, since as a run-time one the decoding would issue on the
+// FP64 pipe for all
+template <int N, typename T, bool UNI, bool VISC, int D, bool OWN_TR = false, bool UPW = false, bool LIMBS = false>
 __device__ __forceinline__ void direction_pass_pm(const StageArgs &A, const DevTables<T> &tb,
                                                   const T (&U)[N], T nlo, T nhi, T dnlo, T dnhi, bool blo,
                                                   bool bhi, const FacePM<T> &pm, const T *vt, int vstride,
@@ -330,16 +335,14 @@ __device__ __forceinline__ void direction_pass_pm(const StageArgs &A, const DevT
 {
   constexpr int NF = N * N;
   static_assert(!UPW || (OWN_TR && !VISC), "the upwind form takes its face values from the caller");
-  // vt at point q of the pencil (limbs: the cell geometry of the block
-  // fixed-point kernels, whose cells outside their window run here)
+  // vt at point q of the pencil
   auto vtq = [&](int q) -> T {
-    if constexpr (sizeof(T) == sizeof(double) && !VISC)
-      if (A.vt_limbs)
-        {
-          const double w = vt[q * vstride];
-          return ((double)__double2loint(w) * 536870912.0 + (double)__double2hiint(w)) *
-                 __hiloint2double((vtop - 57) << 20, 0);
-        }
+    if constexpr (LIMBS)
+      {
+        const double w = vt[q * vstride];
+        return ((double)__double2loint(w) * 536870912.0 + (double)__double2hiint(w)) *
+               __hiloint2double((vtop - 57) << 20, 0);
+      }
     return vt[q * vstride];
   };
   T ulo, uhi;
@@ -509,14 +512,14 @@ __device__ __forceinline__ void direction_pass_pm(const StageArgs &A, const DevT
     }
 }
 
-template <int N, typename T, bool UNI, bool VISC, int D, bool OWN_TR = false>
+template <int N, typename T, bool UNI, bool VISC, int D, bool OWN_TR = false, bool LIMBS = false>
 __device__ __forceinline__ void direction_pass(const StageArgs &A, const DevTables<T> &tb,
                                                const T (&U)[N], T nlo, T nhi, T dnlo, T dnhi, bool blo,
                                                bool bhi, int fq, const T *Flo, const T *Fhi, const T *vt,
                                                int vstride, T (&out)[N], T tr_lo = T(0), T tr_hi = T(0),
                                                T dtr_lo = T(0), T dtr_hi = T(0), int vtop = 0)
 {
-  direction_pass_pm<N, T, UNI, VISC, D, OWN_TR>(A, tb, U, nlo, nhi, dnlo, dnhi, blo, bhi,
+  direction_pass_pm<N, T, UNI, VISC, D, OWN_TR, false, LIMBS>(A, tb, U, nlo, nhi, dnlo, dnhi, blo, bhi,
                                                 face_pm<T, UNI, D>(A, Flo, Fhi, fq), vt, vstride, out, tr_lo,
                                                 tr_hi, dtr_lo, dtr_hi, vtop);
 }
@@ -604,7 +607,7 @@ __device__ __forceinline__ void geometry_async(const StageArgs &A, long long cel
 // One CTA's work: cells cell0 .. cell0 + C - 1 of the mesh described by A,
 // with the dynamic shared memory of the launch.  Shared by the single-mesh
 // kernel and the batched multi-mesh kernel of the serving loop.
-template <int N, typename T, bool UNI, bool VISC>
+template <int N, typename T, bool UNI, bool VISC, bool LIMBS = false>
 __device__ __forceinline__ void stage_cta(const StageArgs &A, const long long cell0, unsigned char *smem_raw,
                                           unsigned cell_mask = ~0u)
 {
@@ -805,11 +808,11 @@ __device__ __forceinline__ void stage_cta(const StageArgs &A, const long long ce
       for (int k = 0; k < N; ++k)
         p[k] = U[k];
       const T *F = faces(cl, 0), *Fh = faces(cl, 1);
-      direction_pass<N, T, UNI, VISC, 0>(A, tb, U, Nb[(cl * 6 + 0) * NF + r], Nb[(cl * 6 + 1) * NF + r],
+      direction_pass<N, T, UNI, VISC, 0, false, LIMBS>(A, tb, U, Nb[(cl * 6 + 0) * NF + r], Nb[(cl * 6 + 1) * NF + r],
                                          VISC ? Nd[(cl * 6 + 0) * NF + r] : T(0),
                                          VISC ? Nd[(cl * 6 + 1) * NF + r] : T(0),
                                          s_nbr[cl * 6 + 0] < 0, s_nbr[cl * 6 + 1] < 0, r,
-                                   F, Fh, Gb + cl * 4 * NQ + N * r, 1, out, T(0), T(0), T(0), T(0), vt_top(A, cell0 + cl));
+                                   F, Fh, Gb + cl * 4 * NQ + N * r, 1, out, T(0), T(0), T(0), T(0), vt_top<LIMBS>(A, cell0 + cl));
       T *z = Qb + cl * NQ + N * r;
 #pragma unroll
       for (int k = 0; k < N; ++k)
@@ -828,12 +831,12 @@ __device__ __forceinline__ void stage_cta(const StageArgs &A, const long long ce
       for (int k = 0; k < N; ++k)
         U[k] = p[k * N];
       const T *F = faces(cl, 2), *Fh = faces(cl, 3);
-      direction_pass<N, T, UNI, VISC, 1>(A, tb, U, Nb[(cl * 6 + 2) * NF + r], Nb[(cl * 6 + 3) * NF + r],
+      direction_pass<N, T, UNI, VISC, 1, false, LIMBS>(A, tb, U, Nb[(cl * 6 + 2) * NF + r], Nb[(cl * 6 + 3) * NF + r],
                                          VISC ? Nd[(cl * 6 + 2) * NF + r] : T(0),
                                          VISC ? Nd[(cl * 6 + 3) * NF + r] : T(0),
                                          s_nbr[cl * 6 + 2] < 0, s_nbr[cl * 6 + 3] < 0, r,
                                    F, Fh, Gb + (cl * 4 + 1) * NQ + off, N, out, T(0), T(0), T(0), T(0),
-                                   vt_top(A, cell0 + cl));
+                                   vt_top<LIMBS>(A, cell0 + cl));
       T *z = Qb + cl * NQ + off;
 #pragma unroll
       for (int k = 0; k < N; ++k)
@@ -852,11 +855,11 @@ __device__ __forceinline__ void stage_cta(const StageArgs &A, const long long ce
         U[k] = p[k * NF];
       const T *F = faces(cl, 4), *Fh = faces(cl, 5);
       const T *G = Gb + cl * 4 * NQ;
-      direction_pass<N, T, UNI, VISC, 2>(A, tb, U, Nb[(cl * 6 + 4) * NF + r], Nb[(cl * 6 + 5) * NF + r],
+      direction_pass<N, T, UNI, VISC, 2, false, LIMBS>(A, tb, U, Nb[(cl * 6 + 4) * NF + r], Nb[(cl * 6 + 5) * NF + r],
                                          VISC ? Nd[(cl * 6 + 4) * NF + r] : T(0),
                                          VISC ? Nd[(cl * 6 + 5) * NF + r] : T(0),
                                          s_nbr[cl * 6 + 4] < 0, s_nbr[cl * 6 + 5] < 0, r,
-                                   F, Fh, G + 2 * NQ + r, NF, out, T(0), T(0), T(0), T(0), vt_top(A, cell0 + cl));
+                                   F, Fh, G + 2 * NQ + r, NF, out, T(0), T(0), T(0), T(0), vt_top<LIMBS>(A, cell0 + cl));
       T *z = Qb + cl * NQ + r;
       if (A.mode != kModeVmult)
         {
