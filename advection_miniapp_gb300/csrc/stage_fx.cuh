@@ -42,7 +42,7 @@ struct FxShape
   static_assert(C * N * N <= THREADS && C <= 32, "one pencil per thread and a bit per cell");
   // U and Z [C][NQ], field geometry [C][4][NQ], the block maxima and the mask
   static constexpr int OWN  = (UNI ? 2 : 6) * C * N * N * N * 8 + (2 * C + 1) * 4;
-  static constexpr int BIN  = GaussShape<N, double, UNI, false, TR>::SMEM;
+  static constexpr int BIN  = GaussShape<N, double, UNI, false, TR, !UNI>::SMEM;
   static constexpr int SMEM = OWN > BIN ? OWN : BIN;
   static_assert(2 * C * N * N * N * 8 % 16 == 0, "cp.async destinations need 16-byte alignment");
 };

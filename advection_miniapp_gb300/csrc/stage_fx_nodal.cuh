@@ -10,10 +10,12 @@
 // values; each neighbour face layer by itself; the cell's fluxes with vt U (as
 // stage_fx_cta); the cell's result before S^-1.  Face values become binary64
 // for the flux, Z for 1 / det J, and the result for the update.
-// Bound: integer issue and the latencies between its eleven barriers.
-// Measured on GB300 against the binary64 kernel: five perform_stage calls on
-// 32^3 curved cells of degree 4 1.02 instead of 2.92 ms, apply on 17 x 13 x 11
-// curved cells of degree 6 172 instead of 268 us.
+// Bound: integer issue (48 % of the slots) and the latencies between its
+// eleven barriers at six resident CTAs (degree 4).  Measured on GB300 against
+// the binary64 kernel: five perform_stage calls on 32^3 curved cells of degree 4
+// 0.91 instead of 2.92 ms, apply on 17 x 13 x 11 curved cells of degree 6 142 instead
+// of 268 us; with the binary64 path's staged face coefficients in the same shared
+// memory (four CTAs, one at degree 6) 1.01 ms and 172 us.
 // A cell with a block outside the window of exponents is left to the binary64
 // kernel afterwards, cell by cell.
 #pragma once
@@ -33,7 +35,8 @@ struct FxNodalShape
   // U, Z [C][NQ], neighbour layers [C][6][NF], geometry [C][4][NQ], the block
   // maxima (cell, layers, flux, result), neighbours and faces, the mask
   static constexpr int OWN = ((UNI ? 2 : 6) * C * N * N * N + 6 * C * N * N) * 8 + (4 * C + 6 * C + 12 * C + 1) * 4;
-  static constexpr int BIN  = SH::SMEM;
+  // the binary64 path without staged face coefficients
+  static constexpr int BIN  = SH::SMEM - (UNI ? 0 : 12 * C * N * N * 8);
   static constexpr int SMEM = OWN > BIN ? OWN : BIN;
   static_assert((2 * C * N * N * N + 6 * C * N * N) % 2 == 0, "cp.async destinations need 16-byte alignment");
 };

@@ -35,7 +35,9 @@
 
 namespace adv
 {
-template <int N, typename T, bool UNI, bool VISC, bool TR>
+// LIMBS: the binary64 path of a block fixed-point kernel, which reads geometry and
+// face coefficients from global memory to fit that kernel's shared memory
+template <int N, typename T, bool UNI, bool VISC, bool TR, bool LIMBS = false>
 struct GaussShape
 {
   using SH                     = StageShape<N, T, UNI, VISC>;
@@ -68,8 +70,8 @@ struct GaussShape
   // of geometry: +3.6 % on 64^3 curved cells of degree 4 at 7 CTAs per SM).
   // The other advection kernels keep staging it (measured 7 % / 4 % slower
   // without).
-  static constexpr bool GEO_GLOBAL   = VISC || (TR && !UNI && sizeof(T) == sizeof(double));
-  static constexpr bool FACES_GLOBAL = !UNI && (TR || VISC || sizeof(T) == sizeof(float));
+  static constexpr bool GEO_GLOBAL   = LIMBS || VISC || (TR && !UNI && sizeof(T) == sizeof(double));
+  static constexpr bool FACES_GLOBAL = !UNI && (LIMBS || TR || VISC || sizeof(T) == sizeof(float));
   static constexpr int  FB_VALUES    = UNI || FACES_GLOBAL ? 0 : 12 * C * N * N;
   static constexpr int  GB_VALUES    = UNI || GEO_GLOBAL ? 0 : 4 * C * N * N * N;
   // viscous: Nd [C][6][NF] neighbour normal derivatives
@@ -143,7 +145,7 @@ __device__ __forceinline__ void stage_gauss_cta(const StageArgs &A, const long l
   constexpr int NT = SH::THREADS;
   T   *Ub     = reinterpret_cast<T *>(smem_raw); // [C][NQ] Gauss-point values of r_in
   T   *Qb     = Ub + C * NQ;                     // [C][NQ] x and y contributions to Z
-  using GS                 = GaussShape<N, T, UNI, VISC, TR>;
+  using GS                 = GaussShape<N, T, UNI, VISC, TR, LIMBS>;
   constexpr bool FG        = GS::FACES_GLOBAL;
   constexpr int  TRW       = GS::TRW;
   constexpr bool TG        = GS::TG;

@@ -620,7 +620,9 @@ __device__ __forceinline__ void stage_cta(const StageArgs &A, const long long ce
   T   *Qb     = Ub + C * NQ;                     // [C][NQ] accumulated Z, then k
   T   *Nb     = Qb + C * NQ;                     // [C][6][NF] neighbour face values
   T   *Gb     = Nb + C * 6 * NF;                 // field: [C][4][NQ] cell geometry
-  constexpr bool FG = SH::FACES_GLOBAL;
+  // (cells outside a block fixed-point kernel's window, LIMBS, read the face
+  // coefficients from global memory too, to fit that kernel's shared memory)
+  constexpr bool FG = SH::FACES_GLOBAL || LIMBS;
   T   *Fb     = Gb + (UNI ? 0 : C * 4 * NQ);     // field: [C][6][2][NF] face coefficients (staged unless FG)
   T   *Nd     = Fb + (UNI || FG ? 0 : C * 12 * NF); // viscous: [C][6][NF] neighbour normal derivatives
   int *s_nbr  = reinterpret_cast<int *>(Nd + (VISC ? C * 6 * NF : 0)); // [C][6] neighbour or -1
