@@ -22,7 +22,7 @@
 namespace adv
 {
 // resident threads per SM the register allocation allows for (80 registers a
-// thread); measured on 64^3 curved cells of degree 4, 4 steps: 16.61 ms with
+// thread); measured with the first staged version of the collocation kernel on 64^3 curved cells of degree 4, 4 steps: 16.61 ms with
 // 768, 16.67 with 640, 16.54 with 896, 18.72 with 512; 29 x 23 x 37 affine
 // cells of degree 2: 686, 730, 682 and 733 us
 constexpr int kFxThreadsPerSM = 768;

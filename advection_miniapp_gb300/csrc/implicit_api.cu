@@ -27,6 +27,7 @@ struct adv_solver
   int         precond_precision = 1;
   int64_t     n                 = 0;
   double     *V = nullptr, *Z = nullptr, *w = nullptr, *tmp = nullptr, *b = nullptr;
+  double     *jxw = nullptr; // field geometry: JxW at the Gauss points (null: not enough memory)
   double     *d_small    = nullptr; // [coef1 (m+1) | coef2 (m+1) | norm | y (m)]
   double     *d_partials = nullptr;
   void       *d_tables   = nullptr;
@@ -51,11 +52,12 @@ int alloc(void **p, size_t bytes, int64_t &count)
 // coefficients on the Gauss-point basis (the collocation-form stage kernel,
 // no interpolation or integration sweeps); else both are on the nodal basis
 int launch_vmult(adv_handle *h, const double *src, double *dst, double mass_factor, double t, cudaStream_t s,
-                 bool gauss = false)
+                 bool gauss = false, const double *jxw = nullptr)
 {
   adv::StageArgs A = adv::detail::base_args(*h, t);
   A.mode           = adv::kModeVmult;
   A.gauss          = gauss ? 1 : 0;
+  A.jxw            = jxw;
   A.r_in           = src;
   A.r_out          = dst;
   A.mass_factor    = mass_factor;
@@ -160,6 +162,27 @@ int adv_solver_create(adv_handle *h, int restart, int precond_precision, adv_sol
       adv_solver_destroy(S);
       return rc;
     }
+  // JxW for the Gauss-basis operator (the legacy stream orders it before any
+  // blocking stream; other streams wait for the synchronisation)
+  if (h->fx_ok && !h->mesh.uniform)
+    {
+      if (cudaMalloc((void **)&S->jxw, nb) != cudaSuccess)
+        {
+          cudaGetLastError(); // the operator divides by 1 / det J instead
+          S->jxw = nullptr;
+        }
+      else
+        {
+          S->bytes += (int64_t)nb;
+          if (adv::launch_gauss_mass_lincomb(h->mesh.n, S->jxw, 1.0, nullptr, 0.0, nullptr, h->mesh.n_cells,
+                                             static_cast<const double *>(h->d_cell_geo), 0.0, nullptr) != cudaSuccess ||
+              cudaStreamSynchronize(nullptr) != cudaSuccess)
+            {
+              adv_solver_destroy(S);
+              return fail(ADV_ERR_CUDA, "JxW of the implicit solver");
+            }
+        }
+    }
   // FDM tables per sign: [VWr VWi Vr Vi lr li]
   const int           n = t.n, per = 4 * n * n + 2 * n;
   std::vector<double> tab(2 * per);
@@ -209,6 +232,7 @@ int adv_solver_destroy(adv_solver *S)
   cudaFree(S->Z);
   cudaFree(S->w);
   cudaFree(S->tmp);
+  cudaFree(S->jxw);
   cudaFree(S->b);
   cudaFree(S->d_small);
   cudaFree(S->d_partials);
@@ -330,7 +354,7 @@ int fgmres(adv_solver *S, double mass_factor, double t, const double *rhs, doubl
   while (true)
     {
       // r = rhs - A x into V_0
-      if (int e = launch_vmult(h, x, S->w, mass_factor, t, s, gauss))
+      if (int e = launch_vmult(h, x, S->w, mass_factor, t, s, gauss, S->jxw))
         return e;
       ADV_CUDA(adv::launch_lincomb(S->V, 1.0, rhs, -1.0, S->w, n, s));
       double beta = 0.0;
@@ -370,7 +394,7 @@ int fgmres(adv_solver *S, double mass_factor, double t, const double *rhs, doubl
           double *vj = S->V + j * n, *zj = S->Z + j * n;
           if (int e = precondition(S, vj, zj, mass_factor, t, s, gauss))
             return e;
-          if (int e = launch_vmult(h, zj, S->w, mass_factor, t, s, gauss))
+          if (int e = launch_vmult(h, zj, S->w, mass_factor, t, s, gauss, S->jxw))
             return e;
           // classical Gram-Schmidt, twice
           ADV_CUDA(adv::launch_multi_dot(S->V, n, j + 1, S->w, n, S->d_partials, c1, s));

@@ -644,7 +644,7 @@ cudaError_t launch_lincomb(double *dst, double a, const double *x, double b, con
 
 namespace
 {
-// dst = JxW (a x + b y) at every Gauss point (y may be null), grid-stride over
+// dst = JxW (a x + b y) at every Gauss point (y may be null; a null x is 1), grid-stride over
 // the points; JxW = w_q / idet_q from the cell geometry, or w_q V (uniform)
 template <int N>
 __global__ void __launch_bounds__(kVecThreads)
@@ -660,7 +660,7 @@ __global__ void __launch_bounds__(kVecThreads)
       const int       q   = (int)(e - c * NQ);
       const double    w   = tb.gw[q % N] * tb.gw[(q / N) % N] * tb.gw[q / (N * N)];
       const double    jxw = cell_geo ? w / __ldg(cell_geo + c * 4 * NQ + 3 * NQ + q) : w * vol;
-      double          v   = a * __ldg(x + e);
+      double          v   = x ? a * __ldg(x + e) : a;
       if (y)
         v = fma(b, __ldg(y + e), v);
       dst[e] = jxw * v;

@@ -54,6 +54,7 @@ struct StageArgs
   // its upwind cell; stages read and write only those (see stage_gauss.cuh)
   int           upwind_tr;
   double        mass_factor; // vmult mode: factor of the mass matrix
+  const double *jxw;         // vmult mode, collocation, field case (optional): JxW at every Gauss point
   float         mass_factorf;
   float         volf;        // uniform case: cell volume (det J)
   double        vol;

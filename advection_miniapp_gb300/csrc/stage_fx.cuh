@@ -4,23 +4,23 @@
 // The mathematics, data layout and outputs are those of stage_gauss_cta
 // (stage_gauss.cuh) with a binary64 operator; the volume and lift
 // contractions of the three direction passes, which were 75 % of its FP64
-// instructions, run on the integer pipes.  Per cell: the largest |U| and the
-// largest face flux give the power of two of the block, U is converted once
-// to limb pairs in shared memory, each pass multiplies its pencil with vt
-// (mantissa products), contracts it with Dw and the lifts, and adds 64-bit
+// instructions, run on the integer pipes, and so do the fluxes.  Per cell: the
+// largest |U| and the largest face flux give the power of two of the block, U is
+// converted once to limb pairs in shared memory, each pass multiplies its pencil
+// with vt (stored as limbs), contracts it with Dw and the lifts, and adds 64-bit
 // integers into Z, which becomes binary64 again once, in the Runge-Kutta
-// update.  Face values, fluxes, 1 / det J, the update and the next face
-// traces stay binary64.
+// update.  1 / det J, the update and the next face traces stay binary64.
 //
-// Bound: the latency of the two dependent reads of a CTA (coefficients, then
-// the upwind traces), then the FP64 pipe (9 instead of 27 instructions per
-// point: fluxes, 1 / det J, update, traces) and HBM; the geometry comes by
-// cp.async behind the fluxes and the solution ahead of the last pass.
-// Measured on GB300 against the binary64 kernel: 64^3 curved cells of degree
-// 4, LSRK(5,4): 16.6 instead of 36.1 ms per 4 steps (with both changes of
-// basis); 29 x 23 x 37 affine cells of degree 2, 4 steps of the 7-stage scheme:
-// 0.69 instead of 1.94 ms; 512 affine cells of degree 3, one step: 56 instead
-// of 76 us.
+// Bound: FP64 issue (6.5 instead of 27 instructions per point: 1 / det J,
+// update, traces) and integer issue, both near 60 %, at 63 % of the HBM
+// bandwidth on curved cells; the geometry comes by cp.async behind the fluxes and
+// the solution ahead of the last pass.  Measured on GB300 against the binary64
+// kernel: 64^3 curved cells of degree 4, LSRK(5,4): 12.6 instead of 36.1 ms per 4 steps
+// (with both changes of basis); 37 x 23 x 29 affine cells of degree 2, 4 steps of the
+// 7-stage scheme: 0.54 instead of 1.94 ms; 512 affine cells of degree 3, one step: 44
+// instead of 76 us.  On the way (4 steps at 64^3): geometry read in the passes 25.6 ms,
+// staged by cp.async with one trace read per face point 16.6, fluxes as integer
+// products 13.8, no predicated FP64 code 12.6.
 //
 // Cells whose block leaves the safe window of exponents (infinities, NaN,
 // magnitudes outside about 2^-400 .. 2^600) are left out here and computed
@@ -330,14 +330,30 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
         kd[k] = fx_to_double(Qb[off + k * NF] + out[k], ez);
       if (!TR && A.mode == kModeVmult)
         {
-          // implicit operator in weak form: JxW (c U - bracket), as stage_gauss_cta
-#pragma unroll
-          for (int k = 0; k < N; ++k)
+          // implicit operator in weak form: JxW (c U - bracket), as
+          // stage_gauss_cta; with JxW given, without the division by 1 / det J (half
+          // of this mode's FP64 instructions: 135 instead of 187 us on 32^3 curved
+          // cells of degree 4)
+          if (!UNI && A.jxw)
             {
-              const double wq = tb.gw[r % N] * tb.gw[r / N] * tb.gw[k];
-              const double br = A.out_scale * kd[k], u = __ldg(A.r_in + gb + k * NF);
-              A.r_out[gb + k * NF] = UNI ? wq * A.vol * (A.mass_factor * u - br)
-                                         : wq * (A.mass_factor * u / G[3 * NQ + r + k * NF] - br);
+              const double wxy = tb.gw[r % N] * tb.gw[r / N];
+#pragma unroll
+              for (int k = 0; k < N; ++k)
+                U[k] = (A.mass_factor * __ldg(A.r_in + gb + k * NF)) * __ldg(A.jxw + gb + k * NF);
+#pragma unroll
+              for (int k = 0; k < N; ++k)
+                A.r_out[gb + k * NF] = fma(-(wxy * tb.gw[k]), A.out_scale * kd[k], U[k]);
+            }
+          else
+            {
+#pragma unroll
+              for (int k = 0; k < N; ++k)
+                {
+                  const double wq = tb.gw[r % N] * tb.gw[r / N] * tb.gw[k];
+                  const double br = A.out_scale * kd[k], u = __ldg(A.r_in + gb + k * NF);
+                  A.r_out[gb + k * NF] = UNI ? wq * A.vol * (A.mass_factor * u - br)
+                                             : wq * (A.mass_factor * u / G[3 * NQ + r + k * NF] - br);
+                }
             }
         }
       else

@@ -149,7 +149,7 @@ def fp_work_per_cell(n, curved=True, stage=True, collocation=False, traces=False
 # kernels, from ncu captures of the 40^3 curved degree-4 case (8,000,000 DoFs,
 # vectors and geometry larger than L2; profiles/ has the commands), scaled to
 # the workload by the DoF count
-NCU_TRAFFIC_PER_DOF = {"fp64": (531.901184e6 + 145.704960e6) / 8.0e6, "fp32": (297.173248e6 + 95.730432e6) / 8.0e6,
+NCU_TRAFFIC_PER_DOF = {"fp64": (528.244992e6 + 146.566912e6) / 8.0e6, "fp32": (297.173248e6 + 95.730432e6) / 8.0e6,
                        # FP32 increment stage (stage_gauss_kernel<5, float, ..., INC>), the block's
                        # dominant kernel: 19 of the 21 launches of a 4-step block
                        "fp32_increment": (309.134336e6 + 67.868928e6) / 8.0e6}
@@ -574,9 +574,8 @@ def ours(args):
              + fp_work_per_cell(n, stage=False, collocation=True, traces=True, upwind=True)[1]) / STAGES
     flops32 = (4 * fp_work_per_cell(n)[1] + fp_work_per_cell(n, stage=False)[1]) / STAGES
     vec_bytes_launch = bytes_per_dof_step() / STAGES * n_dofs
-    # FP64 instructions of any kind (FMA, add, mul) take one issue slot of the
-    # FP64 pipe; expressed as FMA-equivalent TFLOP/s (2 flops per slot) they
-    # compare with the measured FMA peak
+    # the stage's FP64 instructions in binary64 arithmetic as FMA-equivalent
+    # TFLOP/s (2 flops per issue slot), for comparison with the measured FMA peak
     achieved64 = 2 * inst * n_cells / launch64 / 1e12
     algorithmic64 = flops * n_cells / launch64 / 1e12
     achieved32_hbm = vec_bytes_launch / launch32 / 1e9
@@ -619,21 +618,19 @@ def ours(args):
         "config": config_dict(), "precision": "FP64 operator, FP64 vectors",
         "parallelism": f"replicas x{world}" if world > 1 else "single GPU",
         "rel_l2_error": r64["rel_l2"],
-        "roofline": {"bound": "fp64", "achieved": round(achieved64, 4), "peak": round(fp64_peak, 4),
-                     "unit": "TFLOP/s", "frac": round(achieved64 / fp64_peak, 4),
+        "roofline": {"bound": "hbm", "achieved": round(vec_bytes_launch / launch64 / 1e9 + geo64, 2), "peak": hbm_peak,
+                     "unit": "GB/s", "frac": round((vec_bytes_launch / launch64 / 1e9 + geo64) / hbm_peak, 4),
                      "traffic": traffic(NCU_TRAFFIC_PER_DOF["fp64"], n_dofs),
-                     "form": "collocation with upwind face traces (Gauss-point values inside lsrk_steps)",
-                     "peak_source": "FP64 FMA microbenchmark (adv_measure_fma_peak) on this GPU",
-                     "achieved_definition": "2 x FP64 instructions per second (each FP64 add/mul/FMA takes one "
-                                            "FMA issue slot); algorithmic_tflops counts FMA = 2, add/mul = 1",
-                     "algorithmic_tflops": round(algorithmic64, 4),
-                     "flops_per_cell": flops, "fp64_inst_per_cell": inst,
-                     "fp64_inst_frac": round(inst * n_cells / launch64 / (fp64_peak * 1e12 / 2), 4),
+                     "form": "collocation with upwind face traces (Gauss-point values inside lsrk_steps), "
+                             "contractions in block fixed-point arithmetic on the integer pipes",
+                     "definition": "algorithmic vector and geometry bytes of a stage over its time",
+                     "algorithmic_tflops": round(algorithmic64, 4), "flops_per_cell": flops,
+                     "fp64_model_inst_per_cell": inst,
+                     "fp64_model_tflops": round(achieved64, 4), "fp64_peak_tflops": round(fp64_peak, 4),
+                     "fp64_model_definition": "2 x the FP64 instructions of the same stage in binary64 per second, beside "
+                                              "the measured FMA peak: above it because the contractions do not "
+                                              "run on the FP64 pipe",
                      "fp64_mix_peak": round(fp64_mix_peak, 4),
-                     "frac_of_mix_peak": round(achieved64 / fp64_mix_peak, 4),
-                     "mix_peak_source": "adv_measure_fma_peak(2): 7 FMA, 4 MUL, 3 ADD chains per iteration",
-                     "hbm_achieved_gbs": round(vec_bytes_launch / launch64 / 1e9 + geo64, 2),
-                     "hbm_frac_of_measured": round((vec_bytes_launch / launch64 / 1e9 + geo64) / hbm_peak, 4),
                      "launch_ms": round(launch64 * 1e3, 4)},
         "fp32_operator": {
             "value": round(v32, 4), "unit": "GDoF/s", "speedup_vs_fp64": round(v32 / v64, 3),
