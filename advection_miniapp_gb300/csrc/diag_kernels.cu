@@ -242,7 +242,8 @@ __global__ void __launch_bounds__(kDiagThreads) project_kernel(const __grid_cons
   const double tt = ex.constant_velocity ? 1.0 : t;
 #pragma unroll
   for (int d = 0; d < 3; ++d)
-    ex.velocity[d] = __dmul_rn(g.ex.velocity[d], t);
+    if (ex.constant_velocity)
+      ex.velocity[d] = __dmul_rn(g.ex.velocity[d], t);
   for (long long c = g.cell_begin + blockIdx.x; c < g.n_cells; c += gridDim.x)
     {
       double lo[3];
