@@ -423,9 +423,15 @@ __device__ __forceinline__ void dot_group(const double *__restrict__ v, long lon
 // warp), and the warps' sums wait in shared memory for one barrier at the
 // end.  A fixed order, so results repeat.  Bound: the FP64 pipe (two
 // products per clock and SM).  Measured on GB300 over the 290 calls of two
-// BDF2 steps with 4.1M entries at Courant 8: 14.6 instead of 18.7 ms.
+// BDF2 steps with 4.1M entries at Courant 8: 18.7 ms one vector at a time, 14.6
+// with groups of four, 2.3 less with the last two or three together and one
+// wave of blocks.
 constexpr int kMaxDots = 64;
-__global__ void __launch_bounds__(kVecThreads)
+// resident blocks per SM; the grid is at most one wave of them (a second,
+// partial wave cost 6 % of a BDF2 step at 4.1M entries).  Two BDF2 steps with
+// (dot, axpy) = (3, 6) 29.9 ms, (4, 6) 30.2, (6, 6) 31.1, (4, 8) 30.7, (3, 5) 30.4
+constexpr int kDotBlocks = 3, kAxpyBlocks = 6;
+__global__ void __launch_bounds__(kVecThreads, kDotBlocks)
   multi_dot_kernel(const double *__restrict__ V, long long ld, int m, const double *__restrict__ w, long long n,
                    double *partials)
 {
@@ -449,6 +455,19 @@ __global__ void __launch_bounds__(kVecThreads)
             t += __shfl_xor_sync(0xffffffffu, t, o);
           if ((lane & 7) == 0)
             red[warp][i + (lane >> 3)] = t;
+        }
+      // the last one to three
+      if (mm - i >= 2)
+        {
+          double       s[2];
+          dot_group<2>(V + (i0 + i) * ld, ld, w, first, stride, n, s);
+          const bool   h4 = lane & 16;
+          double       t  = (h4 ? s[1] : s[0]) + __shfl_xor_sync(0xffffffffu, h4 ? s[0] : s[1], 16);
+          for (int o = 8; o > 0; o >>= 1)
+            t += __shfl_xor_sync(0xffffffffu, t, o);
+          if ((lane & 15) == 0)
+            red[warp][i + (lane >> 4)] = t;
+          i += 2;
         }
       for (; i < mm; ++i)
         {
@@ -496,7 +515,7 @@ __global__ void __launch_bounds__(kVecThreads) reduce_partials_kernel(const doub
 }
 
 // w += sign * sum_i coef[i] V_i
-__global__ void __launch_bounds__(kVecThreads)
+__global__ void __launch_bounds__(kVecThreads, kAxpyBlocks)
   multi_axpy_kernel(double *w, const double *__restrict__ V, long long ld, int m, const double *__restrict__ coef,
                     double sign, long long n)
 {
@@ -622,7 +641,7 @@ cudaError_t launch_multi_dot(const double *V, long long ld, int m, const double 
   // and 64 measured 3 % slower over a BDF2 step at 4.1M entries)
   // (at most vec_blocks(n) blocks, the size of the partials)
   const long long want   = (n + 16 * kVecThreads - 1) / (16 * kVecThreads);
-  const int       blocks = (int)std::max<long long>(1, std::min<long long>(want, std::min(vec_blocks(n), 152 * 6)));
+  const int       blocks = (int)std::max<long long>(1, std::min<long long>(want, std::min(vec_blocks(n), 152 * kDotBlocks)));
   multi_dot_kernel<<<blocks, kVecThreads, 0, s>>>(V, ld, m, w, n, partials);
   reduce_partials_kernel<<<m, kVecThreads, 0, s>>>(partials, blocks, m, out);
   return cudaGetLastError();
@@ -631,7 +650,7 @@ cudaError_t launch_multi_dot(const double *V, long long ld, int m, const double 
 cudaError_t launch_multi_axpy(double *w, const double *V, long long ld, int m, const double *coef, double sign,
                               long long n, cudaStream_t s)
 {
-  multi_axpy_kernel<<<vec_blocks(n), kVecThreads, 0, s>>>(w, V, ld, m, coef, sign, n);
+  multi_axpy_kernel<<<std::min(vec_blocks(n), 152 * kAxpyBlocks), kVecThreads, 0, s>>>(w, V, ld, m, coef, sign, n);
   return cudaGetLastError();
 }
 
