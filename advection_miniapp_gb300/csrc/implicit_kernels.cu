@@ -424,12 +424,12 @@ __device__ __forceinline__ void dot_group(const double *__restrict__ v, long lon
 // end.  A fixed order, so results repeat.  Bound: the FP64 pipe (two
 // products per clock and SM).  Measured on GB300 over the 290 calls of two
 // BDF2 steps with 4.1M entries at Courant 8: 18.7 ms one vector at a time, 14.6
-// with groups of four, 2.3 less with the last two or three together and one
-// wave of blocks.
+// with groups of four, 10.1 with the pair and one wave of blocks (below).
 constexpr int kMaxDots = 64;
-// resident blocks per SM; the grid is at most one wave of them (a second,
-// partial wave cost 6 % of a BDF2 step at 4.1M entries).  Two BDF2 steps with
-// (dot, axpy) = (3, 6) 29.9 ms, (4, 6) 30.2, (6, 6) 31.1, (4, 8) 30.7, (3, 5) 30.4
+// Resident blocks per SM; the grid is at most one wave of them, and the last two
+// or three vectors of a product go in a pair.  The two BDF2 steps with (dot,
+// axpy) = (3, 6) 29.9 ms, (4, 6) 30.2, (6, 6) 31.1, (4, 8) 30.7, (3, 5) 30.4;
+// 32.2 with six product blocks, single last vectors and no limit for updates.
 constexpr int kDotBlocks = 3, kAxpyBlocks = 6;
 __global__ void __launch_bounds__(kVecThreads, kDotBlocks)
   multi_dot_kernel(const double *__restrict__ V, long long ld, int m, const double *__restrict__ w, long long n,
