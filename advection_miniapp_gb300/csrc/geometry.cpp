@@ -316,9 +316,10 @@ void compute_geometry(const adv_config &cfg, const Mesh &m, const Tables1D &tb, 
                 outside |= !in_fx_window(out[3 * nq + q]);
                 vol += det * w;
               }
-            // (a cell without velocity: any exponent in the window does)
+            // (a cell without velocity: the window's lowest exponent, which never sets
+            // the scale beside the diffusion coefficients of the SIPG stage)
             outside |= vmax != 0.0 && !in_fx_window(vmax);
-            g.cell_exp[c] = vmax != 0.0 ? std::ilogb(vmax) + 1023 : 1023;
+            g.cell_exp[c] = (vmax != 0.0 ? std::ilogb(vmax) : -200) + 1023;
             for (int d = 0; d < 3; ++d)
               g.fdm_cell[4 * c + d] = vavg[d] / vol;
             g.fdm_cell[4 * c + 3] = 1.0 / vol;

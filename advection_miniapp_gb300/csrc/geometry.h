@@ -65,7 +65,8 @@ struct HostGeometry
   // block fixed-point path: whether the metric is inside its window of
   // exponents (uniform: the largest |cv|; field: vt's largest entry of every
   // cell and every 1 / det J within 2^+-200), and in the field case the biased
-  // binary64 exponent of the largest |vt| of every cell
+  // binary64 exponent of the largest |vt| of every cell (without velocity: that
+  // of 2^-200)
   bool             fx_ok = false;
   std::vector<int> cell_exp;
   // per cell (v0, v1, v2, 1/|K|): JxW-weighted cell average of J^{-1} b and the
