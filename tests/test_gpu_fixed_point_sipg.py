@@ -36,3 +36,17 @@ def test_diffusion_without_velocity(cuda, oracle_mod, adv_lib, nu, edge, degree)
     got, ref = increments(cuda, oracle_mod, adv_lib, cfg, 0.0, diffusive_step(cfg, edge), degree)
     assert np.abs(ref).max() > 0.0
     assert np.abs(got - ref).max() <= TOL * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("degree", [1, 3, 6])
+@pytest.mark.parametrize("nu", [1e-3, 1e-9])
+def test_diffusion_while_the_velocity_reverses(cuda, oracle_mod, adv_lib, nu, degree):
+    """cos(pi t / T) is 6e-17 at t = T / 2; T is so long that dt does not move t."""
+    period = 1e25
+    cfg = dict(degree=degree, n_cells=(3, 2, 3), periodic=0, velocity_type=1, velocity=(1.0, 1.0, 0.3),
+               velocity_period=period, diffusion=nu, initial_condition=1, ic_params=(0.3, 0.5, 0.5, 0.2),
+               boundary_value=0)
+    dt = diffusive_step(cfg, 1.0)
+    assert period / 2 + dt == period / 2
+    got, ref = increments(cuda, oracle_mod, adv_lib, cfg, period / 2, dt, degree)
+    assert np.abs(got - ref).max() <= TOL * np.abs(ref).max()
