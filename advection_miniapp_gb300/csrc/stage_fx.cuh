@@ -164,7 +164,7 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
   unsigned own = 0; // bit j: the own trace of face j is read
   if (mine)
     {
-      unsigned mf = 0, mu = 0;
+      unsigned mf = 0;
       // coefficients of the own and the neighbour's value at face j
       auto co = [&](int j) { return (j & 1) ? P[j] : M[j]; };
       auto cn = [&](int j) { return (j & 1) ? M[j] : P[j]; };
@@ -224,10 +224,7 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
 #pragma unroll
       for (int j = 0; j < 6; ++j)
         mf = max(mf, fx_product_top(fc[j], fv[j]));
-#pragma unroll
-      for (int k = 0; k < N; ++k)
-        mu = max(mu, abs_hi(U[k]));
-      atomicMax(s_eu + cl, mu);
+      atomicMax(s_eu + cl, fx_magnitude(U));
       atomicMax(s_ef + cl, mf);
     }
   __syncthreads();
@@ -235,7 +232,7 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
   // ---- the block's scale: biased exponents of the tops of U, vt U and Z
   Limbs f[6];
   int2  cv[3];
-  bool  live = mine;
+  bool  live = mine, tiny = false;
   int   topz = 0;
   if (mine)
     {
@@ -246,7 +243,9 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
       const bool zero = (mu | mf) == 0;
       topz            = zero ? 1023 : max(eu + topv - 1022, ef);
       live            = eu < 1623 && ef < 1623 && topz > 623;
-      if (!live && r == 0)
+      // (values of magnitude 0 that are not zero: the binary64 path)
+      tiny = mu == 0;
+      if ((!live && r == 0) || (tiny && fx_subnormal(U)))
         atomicOr(s_bad, 1u << cl);
       // U so that vt U is in Z's scale (topu >= eu)
       const int topu = topz - topv + 1022;
@@ -272,6 +271,8 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
   if (!UNI)
     __pipeline_wait_prior(0);
   __syncthreads();
+  if (tiny)
+    live = live && !((*s_bad >> cl) & 1u);
 
   // one direction pass: the pencil at p (stride st) with vt at v (stride st)
   auto pass = [&](const int2 *p, int st, const double *v, const int2 &c, const Limbs &flo, const Limbs &fhi,

@@ -110,26 +110,18 @@ __device__ __forceinline__ void stage_fx_nodal_cta(const StageArgs &A, const lon
           const int     j = cf % 6, d = j >> 1, layer = (j & 1) ? 0 : N - 1;
           const int     base   = d == 0 ? layer + NF * b : d == 1 ? N * layer + NF * b : N * b + NF * layer;
           const double *g      = A.r_in + (long long)s_nbr[cf] * NQ + base;
-          unsigned      m      = 0;
 #pragma unroll
           for (int a = 0; a < N; ++a)
             rows[q][a] = __ldg(g + a * (d == 0 ? N : 1));
-#pragma unroll
-          for (int a = 0; a < N; ++a)
-            m = max(m, abs_hi(rows[q][a]));
-          atomicMax(s_en + cf, m);
+          atomicMax(s_en + cf, fx_magnitude(rows[q]));
         }
     }
   if (mine)
     {
-      unsigned m = 0;
 #pragma unroll
       for (int k = 0; k < N; ++k)
-        {
-          reinterpret_cast<double *>(Ub)[oz + k * NF] = x[k];
-          m                                           = max(m, abs_hi(x[k]));
-        }
-      atomicMax(s_eu + cl, m);
+        reinterpret_cast<double *>(Ub)[oz + k * NF] = x[k];
+      atomicMax(s_eu + cl, fx_magnitude(x));
     }
   __syncthreads();
 
@@ -152,6 +144,9 @@ __device__ __forceinline__ void stage_fx_nodal_cta(const StageArgs &A, const lon
   // ---- S along x (own cell) and along the layers' first tangential direction
   int  top  = 1023;
   bool live = mine && fx_window(s_eu[cl], top);
+  // (values of magnitude 0 that are not zero: the binary64 path)
+  if (live && s_eu[cl] == 0u && fx_subnormal(x))
+    atomicOr(s_bad, 1u << cl);
   if (live)
     {
 #pragma unroll
@@ -170,12 +165,11 @@ __device__ __forceinline__ void stage_fx_nodal_cta(const StageArgs &A, const lon
       if (i < ncell * 6 * N && s_nbr[cf] >= 0)
         {
           int topn;
-          if (!fx_window(s_en[cf], topn))
-            {
-              if (b == 0)
-                atomicOr(s_bad, 1u << (cf / 6));
-              continue;
-            }
+          const bool in = fx_window(s_en[cf], topn);
+          if (s_en[cf] == 0u ? fx_subnormal(rows[q]) : !in && b == 0)
+            atomicOr(s_bad, 1u << (cf / 6));
+          if (!in)
+            continue;
 #pragma unroll
           for (int a = 0; a < N; ++a)
             X[a] = fx_from_double(rows[q][a], topn);
@@ -258,7 +252,6 @@ __device__ __forceinline__ void stage_fx_nodal_cta(const StageArgs &A, const lon
   double F[6];
   if (live)
     {
-      unsigned m = 0;
 #pragma unroll
       for (int d = 0; d < 3; ++d)
         {
@@ -294,10 +287,9 @@ __device__ __forceinline__ void stage_fx_nodal_cta(const StageArgs &A, const lon
                 }
               const double un = Nb[cf * NF + r];
               F[2 * d + s]    = s ? -fma(P, uo[1], M * un) : fma(M, uo[0], P * un);
-              m               = max(m, abs_hi(F[2 * d + s]));
             }
         }
-      atomicMax(s_ef + cl, m);
+      atomicMax(s_ef + cl, fx_magnitude(F));
     }
   if (!UNI)
     __pipeline_wait_prior(0);
@@ -308,6 +300,7 @@ __device__ __forceinline__ void stage_fx_nodal_cta(const StageArgs &A, const lon
   Limbs f[6];
   int2  cv[3];
   int   dz = 0;
+  bool  tiny = false;
   if (live)
     {
       topv = UNI ? (int)(max(max(abs_hi(A.cv[0]), abs_hi(A.cv[1])), abs_hi(A.cv[2])) >> 20) : A.cell_exp[cell0 + cl];
@@ -321,6 +314,9 @@ __device__ __forceinline__ void stage_fx_nodal_cta(const StageArgs &A, const lon
           if (r == 0)
             atomicOr(s_bad, 1u << cl);
         }
+      tiny = mf == 0;
+      if (tiny && fx_subnormal(F))
+        atomicOr(s_bad, 1u << cl);
       dz = min(max(topz - (top3 + topv - 1022), 0), 63);
 #pragma unroll
       for (int j = 0; j < 6; ++j)
@@ -355,6 +351,8 @@ __device__ __forceinline__ void stage_fx_nodal_cta(const StageArgs &A, const lon
         Qb[ox + k] = T[k];
     }
   __syncthreads();
+  if (tiny)
+    live = live && !((*s_bad >> cl) & 1u);
   if (live)
     {
       pass(Ub + oy, N, G + (oy - cl * NQ) + NQ, cv[1], f[2], f[3]);
@@ -368,7 +366,6 @@ __device__ __forceinline__ void stage_fx_nodal_cta(const StageArgs &A, const lon
     {
       pass(Ub + oz, NF, G + 2 * NQ + r, cv[2], f[4], f[5]);
       const int ez = topz - 1022 - 57 + fx_kd<N>() - kFxGuard;
-      unsigned  m  = 0;
 #pragma unroll
       for (int k = 0; k < N; ++k)
         {
@@ -383,9 +380,8 @@ __device__ __forceinline__ void stage_fx_nodal_cta(const StageArgs &A, const lon
             }
           else
             x[k] = UNI ? z : z * G[3 * NQ + r + k * NF];
-          m = max(m, abs_hi(x[k]));
         }
-      atomicMax(s_ez + cl, m);
+      atomicMax(s_ez + cl, fx_magnitude(x));
     }
   __syncthreads();
 

@@ -213,11 +213,8 @@ struct ViscPencil
   bool  ok;
   __device__ __forceinline__ void set(const double (&x)[N])
   {
-    unsigned m = 0;
-#pragma unroll
-    for (int q = 0; q < N; ++q)
-      m = max(m, abs_hi(x[q]));
-    ok = fx_window(m, top);
+    const unsigned m = fx_magnitude(x);
+    ok               = fx_window(m, top) && !(m == 0u && fx_subnormal(x));
 #pragma unroll
     for (int q = 0; q < N; ++q)
       X[q] = fx_from_double(x[q], top);
@@ -299,7 +296,6 @@ __device__ __forceinline__ void stage_fx_visc_cta(const StageArgs &A, const long
       const unsigned c = (unsigned)(cell0 + cl), nx = A.nc[0], ny = A.nc[1];
       const unsigned row = c / nx;
       const int      ix = (int)(c - row * nx), iz = (int)(row / ny), iy = (int)(row - (unsigned)iz * ny);
-      unsigned       mf = 0, mu = 0;
 #pragma unroll
       for (int j = 0; j < 6; ++j)
         {
@@ -348,20 +344,16 @@ __device__ __forceinline__ void stage_fx_visc_cta(const StageArgs &A, const long
           const double k2   = (j & 1) ? A.K2[d] : -A.K2[d];
           F[j]              = fma(k2, n.y + o.y, flux);
           J[j]              = (A.K2[d] * kj) * jump;
-          mf                = max(mf, max(abs_hi(F[j]), abs_hi(J[j])));
         }
-#pragma unroll
-      for (int k = 0; k < N; ++k)
-        mu = max(mu, abs_hi(U[k]));
-      atomicMax(s_eu + cl, mu);
-      atomicMax(s_ef + cl, mf);
+      atomicMax(s_eu + cl, fx_magnitude(U));
+      atomicMax(s_ef + cl, max(fx_magnitude(F), fx_magnitude(J)));
     }
   __syncthreads();
 
   // ---- the block's scale, kFxViscBits above the largest term
   Limbs f[6], jl[6];
   int2  cd[3];
-  bool  live = mine;
+  bool  live = mine, tiny = false;
   int   topz = 0, topw = 0, topvt = 0;
   if (mine)
     {
@@ -381,7 +373,9 @@ __device__ __forceinline__ void stage_fx_visc_cta(const StageArgs &A, const long
       const bool zero = (mu | mf) == 0;
       topz            = (zero ? 1023 : max(eu + topw - 1022, ef)) + kFxViscBits;
       live            = eu < 1623 && ef < 1623 && topz > 623 + kFxViscBits;
-      if (!live && r == 0)
+      // (values of magnitude 0 that are not zero: the binary64 path)
+      tiny = mu == 0 || mf == 0;
+      if ((!live && r == 0) || (mu == 0 && fx_subnormal(U)) || (mf == 0 && (fx_subnormal(F) || fx_subnormal(J))))
         atomicOr(s_bad, 1u << cl);
       const int topu = topz - topw + 1022;
       if (live)
@@ -408,6 +402,8 @@ __device__ __forceinline__ void stage_fx_visc_cta(const StageArgs &A, const long
         }
     }
   __syncthreads();
+  if (tiny)
+    live = live && !((*s_bad >> cl) & 1u);
 
   auto pass = [&](int off, int st, const double *v, int d, long long(&out)[N]) {
     Limbs X[N], V[N];

@@ -75,14 +75,12 @@ __global__ void __launch_bounds__(StageShape<N, double, true, false>::THREADS)
       __syncthreads();
       if (mine)
         {
-          unsigned m = 0;
 #pragma unroll
           for (int k = 0; k < N; ++k)
-            {
-              buf[oz + k * NF] = x[k];
-              m                = max(m, abs_hi(x[k]));
-            }
-          atomicMax(s_max + cl, m);
+            buf[oz + k * NF] = x[k];
+          const unsigned m = fx_magnitude(x);
+          // (1: not zero although of magnitude 0, outside the window)
+          atomicMax(s_max + cl, m == 0u && fx_subnormal(x) ? 1u : m);
         }
       __syncthreads();
       int        top  = 1023;
