@@ -23,7 +23,7 @@
 // products 13.8, no predicated FP64 code 12.6.
 //
 // Cells whose block leaves the safe window of exponents (infinities, NaN,
-// magnitudes outside about 2^-400 .. 2^600) are left out here and computed
+// magnitudes outside about 2^-722 .. 2^600) are left out here and computed
 // by the binary64 path afterwards, cell by cell, so that a cell's result
 // does not depend on its neighbours in the CTA.
 #pragma once
@@ -242,7 +242,7 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
                            : A.cell_exp[cell0 + cl];
       const bool zero = (mu | mf) == 0;
       topz            = zero ? 1023 : max(eu + topv - 1022, ef);
-      live            = eu < 1623 && ef < 1623 && topz > 623;
+      live            = eu < kFxHigh && ef < kFxHigh && topz > kFxLow;
       // (values of magnitude 0 that are not zero: the binary64 path)
       tiny = mu == 0;
       if ((!live && r == 0) || (tiny && fx_subnormal(U)))

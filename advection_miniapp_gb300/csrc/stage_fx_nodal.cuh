@@ -308,7 +308,7 @@ __device__ __forceinline__ void stage_fx_nodal_cta(const StageArgs &A, const lon
       const int      ef = (int)(mf >> 20);
       // (a cell of zeros takes its fluxes' scale)
       topz = s_eu[cl] ? max(top3 + topv - 1022, ef) : mf ? ef : 1023;
-      if (ef >= 1623 || topz <= 623)
+      if (ef >= kFxHigh || topz <= kFxLow)
         {
           live = false;
           if (r == 0)

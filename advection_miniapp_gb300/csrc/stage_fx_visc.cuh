@@ -372,7 +372,7 @@ __device__ __forceinline__ void stage_fx_visc_cta(const StageArgs &A, const long
         }
       const bool zero = (mu | mf) == 0;
       topz            = (zero ? 1023 : max(eu + topw - 1022, ef)) + kFxViscBits;
-      live            = eu < 1623 && ef < 1623 && topz > 623 + kFxViscBits;
+      live            = eu < kFxHigh && ef < kFxHigh && topz > kFxLow + kFxViscBits;
       // (values of magnitude 0 that are not zero: the binary64 path)
       tiny = mu == 0 || mf == 0;
       if ((!live && r == 0) || (mu == 0 && fx_subnormal(U)) || (mf == 0 && (fx_subnormal(F) || fx_subnormal(J))))

@@ -18,7 +18,7 @@ namespace
 // kernel writes them.
 // The sweeps run in block fixed point, one power of two per cell (fixed.cuh);
 // a cell outside the window of exponents (infinities, NaN, magnitudes outside
-// 2^-400 .. 2^600) in binary64.  The shared buffer holds binary64 values or
+// 2^-722 .. 2^600) in binary64.  The shared buffer holds binary64 values or
 // limbs, 8 bytes each.  Measured on GB300 at 32^3 cells of degree 4: 30
 // instead of 106 us per change of basis with binary64 sweeps (79 % of the FP64
 // peak); a step through host memory at 48^3 2.53 instead of 2.84 ms.

@@ -4,6 +4,8 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
+TOL = 1e-12
+
 MESHES = {
     "uniform": dict(n_cells=(3, 2, 5)),
     "curved": dict(n_cells=(3, 3, 2), mesh_type=1, deformation=0.07),
@@ -48,3 +50,20 @@ def test_values_below_the_normal_range(cuda, oracle_mod, adv_lib, mesh):
     op.apply(s, d, 0.0)
     ref = o.apply(u0, 0.0)
     assert np.abs(d.cpu().numpy() - ref).max() <= 2.0 ** -9 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("exponent", [-760, -740, -720, -700, -560, -410, -395])
+@pytest.mark.parametrize("mesh", sorted(MESHES))
+def test_blocks_near_the_lower_end_of_the_window(cuda, oracle_mod, adv_lib, mesh, exponent):
+    """Cells of 2^(exponent + 0..24): some blocks inside, some outside the window."""
+    cfg = dict(MESHES[mesh], degree=3)
+    o, op = oracle_mod.Oracle(**cfg), adv_lib.AdvectionOperation(**cfg)
+    rng = np.random.default_rng(2)
+    u0 = (rng.standard_normal((o.n_dofs // 64, 64)) * np.exp2(rng.integers(0, 25, (o.n_dofs // 64, 1)))).reshape(-1)
+    got = np.ldexp(gpu_step(cuda, adv_lib, cfg, np.ldexp(u0, exponent), 1e-3), -exponent)
+    ref = oracle_step(o, u0, 1e-3)
+    assert np.abs(got - ref).max() <= TOL * np.abs(ref).max()
+    s, d = cuda.from_numpy(np.ldexp(u0, exponent)).cuda(), op.initialize_dof_vector()
+    op.apply(s, d, 0.0)
+    ref = o.apply(u0, 0.0)
+    assert np.abs(np.ldexp(d.cpu().numpy(), -exponent) - ref).max() <= TOL * np.abs(ref).max()
