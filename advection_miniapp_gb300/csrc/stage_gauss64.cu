@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(StageShape<N, double, true, false>::THREADS)
     {
 #pragma unroll
       for (int k = 0; k < N; ++k)
-        x[k] = __ldg(g + k * NF);
+        x[k] = g[k * NF];
     }
   // face coefficients decide which traces the first stage reads
   unsigned own = 0;
