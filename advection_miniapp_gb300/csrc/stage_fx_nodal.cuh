@@ -239,7 +239,7 @@ __device__ __forceinline__ void stage_fx_nodal_cta(const StageArgs &A, const lon
   int top3 = top;
   if (live)
     {
-      const int sh = 7 - __clz((int)s_e3[cl]); // |T| < 2^(64 - clz) -> 2^58
+      const int sh = 6 - __clz((int)s_e3[cl]); // |T| = 2 |X| < 2^(64 - clz) -> 2^58
       top3 += sh;
 #pragma unroll
       for (int k = 0; k < N; ++k)
