@@ -67,3 +67,18 @@ def test_blocks_near_the_lower_end_of_the_window(cuda, oracle_mod, adv_lib, mesh
     op.apply(s, d, 0.0)
     ref = o.apply(u0, 0.0)
     assert np.abs(np.ldexp(d.cpu().numpy(), -exponent) - ref).max() <= TOL * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("mesh", ["uniform", "curved"])
+def test_small_cells_keep_their_own_accuracy(cuda, oracle_mod, adv_lib, mesh):
+    """Cells of 2^-470 that no value of 1 reaches within the step's five stages."""
+    cfg = dict(MESHES[mesh], degree=4, n_cells=(16, 2, 2))
+    o = oracle_mod.Oracle(**cfg)
+    u0 = np.random.default_rng(5).standard_normal((4, 16, 125))
+    u0[:, 1:] *= 2.0 ** -470
+    u0 = u0.reshape(-1)
+    ref, got = oracle_step(o, u0, 1e-3).reshape(-1, 125), gpu_step(cuda, adv_lib, cfg, u0, 1e-3).reshape(-1, 125)
+    size = np.abs(ref).max(axis=1)
+    small = size < 2.0 ** -400
+    assert small.sum() >= 4 * 5
+    assert (np.abs(got - ref).max(axis=1) <= TOL * size)[small].all()
