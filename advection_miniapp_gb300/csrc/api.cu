@@ -380,6 +380,14 @@ adv::StageArgs base_args(const adv_handle &h, double t, int prec = -1)
       A.visc       = 1;
       A.adv_scale  = s;
       A.adv_scalef = (float)s;
+      // (not finite: the fluxes send every cell to the binary64 path)
+      int e = 0;
+      if (s == 0.0)
+        e = -900;
+      else if (std::isfinite(s))
+        std::frexp(s, &e);
+      A.adv_exp   = std::max(std::min(e, 0), -900);
+      A.adv_limbs = std::isfinite(s) ? adv::fx_const58(s, 1023 + A.adv_exp) : make_int2(0, 0);
       A.out_scale  = 1.0;
       const double nu = h.cfg.diffusion, V = m.h[0] * m.h[1] * m.h[2];
       for (int d = 0; d < 3; ++d)

@@ -48,6 +48,8 @@ struct StageArgs
   float         K1f[3], K2f[3], cdifff[3];
   double        adv_scale;   // velocity time factor, applied in-kernel when visc != 0
   float         adv_scalef;
+  int           adv_exp;     // |adv_scale| <= 2^adv_exp <= 1, and adv_scale 2^-adv_exp as limbs (fx_const58)
+  int2          adv_limbs;
   // face traces on field geometry without SIPG (FP64): the flux is the
   // upwind one (at every face point one of P, M is zero) with a constant
   // velocity and no skew term, so each face point reads only the trace of

@@ -258,7 +258,7 @@ __device__ __forceinline__ void stage_fx_visc_cta(const StageArgs &A, const long
   constexpr int NF = N * N;
   constexpr int NT = FS::THREADS;
   int2      *Ub    = reinterpret_cast<int2 *>(smem_raw);         // [C][NQ] U as limbs
-  int2      *Sb    = Ub + C * NQ;                                // [C][NQ] s 2^-es U / 2 (es below)
+  int2      *Sb    = Ub + C * NQ;                                // [C][NQ] s 2^-es U / 2 (es = adv_exp)
   long long *Qb    = reinterpret_cast<long long *>(Sb + C * NQ); // [C][NQ] Z, then the next input
   unsigned  *s_eu = reinterpret_cast<unsigned *>(Qb + C * NQ), *s_ef = s_eu + C, *s_bad = s_ef + C;
 
@@ -353,16 +353,15 @@ __device__ __forceinline__ void stage_fx_visc_cta(const StageArgs &A, const long
   // ---- the block's scale, kFxViscBits above the largest term
   Limbs f[6], jl[6];
   int2  cd[3];
-  bool  live = mine, tiny = false;
-  int   topz = 0, topw = 0, topvt = 0;
+  bool  live = mine;
+  int   topz = 0, topw = 0;
   if (mine)
     {
       const unsigned mu = s_eu[cl], mf = s_ef[cl];
       const int      eu = (int)(mu >> 20), ef = (int)(mf >> 20);
-      // the velocity term at its own size, s vt: |s| <= 2^es (a velocity near its
+      // the velocity term at its own size, s vt, |s| <= 2^es (a velocity near its
       // reversal in time would set a unit far above the terms of the cell)
-      const int es = max(min((int)(abs_hi(A.adv_scale) >> 20) - 1022, 0), -900);
-      topw         = A.cell_exp[cell0 + cl] + es;
+      topw = A.cell_exp[cell0 + cl] + A.adv_exp;
       double c2[3];
 #pragma unroll
       for (int d = 0; d < 3; ++d)
@@ -374,19 +373,17 @@ __device__ __forceinline__ void stage_fx_visc_cta(const StageArgs &A, const long
       topz            = (zero ? 1023 : max(eu + topw - 1022, ef)) + kFxViscBits;
       live            = eu < kFxHigh && ef < kFxHigh && topz > kFxLow + kFxViscBits;
       // (values of magnitude 0 that are not zero: the binary64 path)
-      tiny = mu == 0 || mf == 0;
       if ((!live && r == 0) || (mu == 0 && fx_subnormal(U)) || (mf == 0 && (fx_subnormal(F) || fx_subnormal(J))))
         atomicOr(s_bad, 1u << cl);
       const int topu = topz - topw + 1022;
       if (live)
         {
-          const int2 sc = fx_const58(A.adv_scale, 1023 + es); // |s| 2^-es <= 1 < 2
 #pragma unroll
           for (int k = 0; k < N; ++k)
             {
               const Limbs x   = fx_from_double(U[k], topu);
               Ub[oz + k * NF] = make_int2(x.h, x.l);
-              const Limbs s   = fx_times(x, sc); // s 2^-es U / 2: vt takes the factor 2^(es + 1) below
+              const Limbs s   = fx_times(x, A.adv_limbs); // s 2^-es U / 2: vt takes the factor 2^(es + 1) below
               Sb[oz + k * NF] = make_int2(s.h, s.l);
             }
 #pragma unroll
@@ -398,12 +395,10 @@ __device__ __forceinline__ void stage_fx_visc_cta(const StageArgs &A, const long
 #pragma unroll
           for (int d = 0; d < 3; ++d)
             cd[d] = fx_const58(c2[d], topw);
-          topvt = topw - 1 - es;
         }
     }
   __syncthreads();
-  if (tiny)
-    live = live && !((*s_bad >> cl) & 1u);
+  live = live && !((*s_bad >> cl) & 1u);
 
   auto pass = [&](int off, int st, const double *v, int d, long long(&out)[N]) {
     Limbs X[N], V[N];
@@ -415,7 +410,7 @@ __device__ __forceinline__ void stage_fx_visc_cta(const StageArgs &A, const long
     for (int k = 0; k < N; ++k)
       {
         const int2 s = Sb[off + k * st];
-        V[k]         = fx_add(fx_times(V[k], cd[d]), fx_times(Limbs{s.x, s.y}, fx_const58(__ldg(v + k * st), topvt)));
+        V[k]         = fx_add(fx_times(V[k], cd[d]), fx_times(Limbs{s.x, s.y}, fx_const58(__ldg(v + k * st), topw - 1 - A.adv_exp)));
       }
     fx_sweep_visc<N>(fx, fv, V, f[2 * d], f[2 * d + 1], jl[2 * d], jl[2 * d + 1], out);
   };
