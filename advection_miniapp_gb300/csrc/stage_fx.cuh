@@ -271,7 +271,10 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
   if (!UNI)
     __pipeline_wait_prior(0);
   __syncthreads();
-  if (tiny)
+  // (on uniform meshes only where a value may be subnormal: reading the mask in
+  // every launch takes a stage on 512 cells from 6.3 to 7.0 us; on field geometry
+  // the plain read is the faster form, 12.66 against 12.69 ms at 64^3)
+  if (!UNI || tiny)
     live = live && !((*s_bad >> cl) & 1u);
 
   // one direction pass: the pencil at p (stride st) with vt at v (stride st)
