@@ -22,9 +22,14 @@
 namespace adv
 {
 // resident threads per SM the register allocation allows for (80 registers a
-// thread); measured with the first staged version of the collocation kernel on 64^3 curved cells of degree 4, 4 steps: 16.61 ms with
-// 768, 16.67 with 640, 16.54 with 896, 18.72 with 512; 29 x 23 x 37 affine
-// cells of degree 2: 686, 730, 682 and 733 us
+// thread).  One three-stage step with 768 / 640 / 512, in us: upwind field
+// geometry 40^3 degree 4 627 / 656 / 718, 24^3 degree 6 514 / 514 / 510; affine
+// 48^3 degree 2 276 / 289 / 308, 24^3 degree 6 403 / 450 / 451; SIPG 40^3 degree 4
+// 1331 / 1339 / 1434, 32^3 degree 5 1162 / 1275 / 1275; apply 40^3 degree 4 322 / 328 / 360.
+// The variants that read every trace of field geometry spill (180-410 bytes of loads)
+// and still prefer 768 at 3 and 5 points (rotating 48^3 degree 2 370 / 371 / 399,
+// Lax-Friedrichs 40^3 degree 4 915 / 919 / 964), but not at 7 (24^3: 618 / 589 /
+// 589 and 690 / 652 / 653); without traces (BDF2) 512 gives 832 instead of 862.
 constexpr int kFxThreadsPerSM = 768;
 
 struct Limbs
@@ -193,7 +198,7 @@ __device__ __forceinline__ double fx_to_double(long long Z, int e)
 // A product with a value X is kept at 2^(kFxGuard - kd) of X's unit, so
 // that the sum over three directions and six lifts of a cell stays below
 // 2^62: 3 (||Dw||_inf + max_q (|lw0| + |lw1|)) 2^(57 + kFxGuard - kd) is at
-// most 2^61.4 for n = 2..7 (20.8, 39.7, 64.0, 93.9, 129.4, 170.6 for the
+// most 2^61.55 for n = 2..7 (20.8, 39.7, 64.0, 93.9, 129.4, 170.6 for the
 // bracket).
 constexpr int kFxGuard = 2, kFxShift = 1 + kFxGuard;
 template <int N>
@@ -297,11 +302,10 @@ __device__ __forceinline__ void fx_sweep_lift(const FxTables &tb, const Limbs (&
     }
 }
 
-// Biased top exponents of a block inside the window: 2^-722 .. 2^600.  Lower end:
-// with metric factors below 2^200 the block's own values then lie 2^64 above
-// the subnormal ones (which the conversions shift out) and what they add to it
-// is 2^-100 of it, and results of 2^-57 times it and of 1 / det J > 2^-200 are
-// normal numbers.  (It was 2^-400; blocks below run twice, in fixed point
+// Biased top exponents of a block inside the window: 2^-722 .. 2^600.  Lower end,
+// with metric factors within 2^+-200: a subnormal value, which the conversions shift
+// out, adds at most 2^-822 to a block, 2^-100 of it; zeros, converted as 2^-1022, lie
+// 2^64 below the unit; 2^-57 of the block times 1 / det J is a normal number.  (It was 2^-400; blocks below run twice, in fixed point
 // as far as their scale and in binary64.  A blob of width 0.05 on the unit cube
 // has cells of 2^-571: on 40^3 affine cells of degree 2 a step took 214 us, now
 // 166, apply 117, now 74.)

@@ -5,8 +5,12 @@
 // pipes they take about 600 instructions, 10 clocks.  The fraction of a turn
 // is carried to 2^-62, the polynomials (Taylor series on |angle| <= pi/4 and on
 // |x| <= ln 2 / 2, their last terms in binary32) to a few 2^-57 of 1, and the sum
-// of the sine product and the Gaussian is rounded to binary64 once: absolute
-// errors of a few 2^-57 where binary64 commits a few 2^-53.
+// of the sine product and the Gaussian is rounded to binary64 once.  Largest
+// errors in units of 2^-57, over 20,000 points each in 200-bit arithmetic: sine 4.2, sine
+// product 3.6, exponential of a given argument 2.9; the Gaussian 14.7, since its
+// argument 50 r^2 is formed in binary64, and the rounded sum 18.2 (one binary64
+// rounding of a result in [1/2, 1) is 8).  These are absolute: far out the Gaussian
+// keeps few bits of its own.
 #pragma once
 
 #include "fixed.cuh"

@@ -13,7 +13,7 @@
 // Bound: integer issue (48 % of the slots) and the latencies between its
 // eleven barriers at six resident CTAs (degree 4).  Measured on GB300 against
 // the binary64 kernel: five perform_stage calls on 32^3 curved cells of degree 4
-// 0.91 instead of 2.92 ms, apply on 17 x 13 x 11 curved cells of degree 6 142 instead
+// 0.91 instead of 2.92 ms, apply on 17 x 13 x 11 curved cells of degree 6 146 instead
 // of 268 us; with the binary64 path's staged face coefficients in the same shared
 // memory (four CTAs, one at degree 6) 1.01 ms and 172 us.
 // A cell with a block outside the window of exponents is left to the binary64

@@ -26,9 +26,11 @@ namespace adv
 // Tables of the diffusive terms: D as c 2^(57 - kdd) and the split derivative
 // lifts lde, ldo as c 2^(57 - kld).  Their operands are carried 2^kdd and
 // 2^(kld - kd) times larger, so that all terms share the unit of the Dw terms.
-// ||D||_inf / 2^kdd is at most 3.9: with one bit of headroom in the block's
-// scale s vt U - nu V / h^2 D U stays below 2^58, and with one guard bit less than
-// the advection stage the sum over three directions below 2^62.
+// ||D||_inf / 2^kdd is 1.7, 1.3, 2.7, 2.4, 3.9, 2.9 for n = 2..7: with one bit of
+// headroom in the block's scale s vt U - nu V / h^2 D U stays below 2^58.3 (its limbs
+// and sums of two of them within 32 bits: h below 2^30.3, l below 2^30), and with one
+// guard bit less than the advection stage the sum over three directions, lifts
+// included, below 2^61.25 (n = 7).
 template <int N>
 constexpr int fx_kdd()
 {
