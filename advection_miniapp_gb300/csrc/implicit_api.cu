@@ -162,27 +162,6 @@ int adv_solver_create(adv_handle *h, int restart, int precond_precision, adv_sol
       adv_solver_destroy(S);
       return rc;
     }
-  // JxW for the Gauss-basis operator (the legacy stream orders it before any
-  // blocking stream; other streams wait for the synchronisation)
-  if (h->fx_ok && !h->mesh.uniform)
-    {
-      if (cudaMalloc((void **)&S->jxw, nb) != cudaSuccess)
-        {
-          cudaGetLastError(); // the operator divides by 1 / det J instead
-          S->jxw = nullptr;
-        }
-      else
-        {
-          S->bytes += (int64_t)nb;
-          if (adv::launch_gauss_mass_lincomb(h->mesh.n, S->jxw, 1.0, nullptr, 0.0, nullptr, h->mesh.n_cells,
-                                             static_cast<const double *>(h->d_cell_geo), 0.0, nullptr) != cudaSuccess ||
-              cudaStreamSynchronize(nullptr) != cudaSuccess)
-            {
-              adv_solver_destroy(S);
-              return fail(ADV_ERR_CUDA, "JxW of the implicit solver");
-            }
-        }
-    }
   // FDM tables per sign: [VWr VWi Vr Vi lr li]
   const int           n = t.n, per = 4 * n * n + 2 * n;
   std::vector<double> tab(2 * per);
@@ -219,6 +198,28 @@ int adv_solver_create(adv_handle *h, int restart, int precond_precision, adv_sol
     {
       adv_solver_destroy(S);
       return rc;
+    }
+  // JxW for the Gauss-basis operator, after everything the solver cannot do
+  // without (the legacy stream orders it before any blocking stream; other
+  // streams wait for the synchronisation)
+  if (h->fx_ok && !h->mesh.uniform)
+    {
+      if (cudaMalloc((void **)&S->jxw, nb) != cudaSuccess)
+        {
+          cudaGetLastError(); // the operator divides by 1 / det J instead
+          S->jxw = nullptr;
+        }
+      else
+        {
+          S->bytes += (int64_t)nb;
+          if (adv::launch_gauss_mass_lincomb(h->mesh.n, S->jxw, 1.0, nullptr, 0.0, nullptr, h->mesh.n_cells,
+                                             static_cast<const double *>(h->d_cell_geo), 0.0, nullptr) != cudaSuccess ||
+              cudaStreamSynchronize(nullptr) != cudaSuccess)
+            {
+              adv_solver_destroy(S);
+              return fail(ADV_ERR_CUDA, "JxW of the implicit solver");
+            }
+        }
     }
   *out = S;
   return ADV_OK;
