@@ -84,7 +84,14 @@ static __device__ __noinline__ double boundary_value(const StageArgs &A, int d, 
   return exact_value(A.ex, x[0], x[1], x[2], A.t);
 }
 
-template <int N, bool UNI, bool TR, bool UPW>
+// LATE: low words are looked at only in blocks of magnitude 0, after the scale, and
+// the mask of cells left out is read again; else they join the maximum of every
+// block.  The first for the uniform launches of one mesh (a stage on 512 cells of
+// degree 3 6.4 us, 6.8 with the second form, 6.4 without the check), the second for
+// field geometry (64^3 curved cells of degree 4, 4 steps 12.62 ms, 12.65 with
+// the first, 12.61 without) and the batched launches (a burst of 16 requests
+// 48.3 ms, 49.3-50.3 with the first, which spills at 7 points, 48.4 without).
+template <int N, bool UNI, bool TR, bool UPW, bool LATE = false>
 __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long cell0, unsigned char *smem_raw)
 {
   using FS         = FxShape<N, UNI, TR>;
@@ -224,7 +231,7 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
 #pragma unroll
       for (int j = 0; j < 6; ++j)
         mf = max(mf, fx_product_top(fc[j], fv[j]));
-      atomicMax(s_eu + cl, fx_magnitude(U));
+      atomicMax(s_eu + cl, LATE ? fx_magnitude(U) : fx_magnitude(U) | (unsigned)fx_subnormal(U));
       atomicMax(s_ef + cl, mf);
     }
   __syncthreads();
@@ -244,7 +251,7 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
       topz            = zero ? 1023 : max(eu + topv - 1022, ef);
       live            = eu < kFxHigh && ef < kFxHigh && topz > kFxLow;
       // (values of magnitude 0 that are not zero: the binary64 path)
-      tiny = mu == 0;
+      tiny = LATE && mu == 0;
       if ((!live && r == 0) || (tiny && fx_subnormal(U)))
         atomicOr(s_bad, 1u << cl);
       // U so that vt U is in Z's scale (topu >= eu)
@@ -271,10 +278,7 @@ __device__ __forceinline__ void stage_fx_cta(const StageArgs &A, const long long
   if (!UNI)
     __pipeline_wait_prior(0);
   __syncthreads();
-  // (on uniform meshes only where a value may be subnormal: reading the mask in
-  // every launch takes a stage on 512 cells from 6.3 to 7.0 us; on field geometry
-  // the plain read is the faster form, 12.66 against 12.69 ms at 64^3)
-  if (!UNI || tiny)
+  if (tiny)
     live = live && !((*s_bad >> cl) & 1u);
 
   // one direction pass: the pencil at p (stride st) with vt at v (stride st)
@@ -452,7 +456,7 @@ __global__ void __launch_bounds__(FxShape<N, UNI, TR>::THREADS, kFxThreadsPerSM 
   stage_fx_kernel(const __grid_constant__ StageArgs A)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  stage_fx_cta<N, UNI, TR, UPW>(A, A.cell_begin + (long long)blockIdx.x * FxShape<N, UNI, TR>::C, smem_raw);
+  stage_fx_cta<N, UNI, TR, UPW, UNI>(A, A.cell_begin + (long long)blockIdx.x * FxShape<N, UNI, TR>::C, smem_raw);
 }
 
 template <int N, bool UNI, bool TR, bool UPW = false>
